@@ -28,7 +28,7 @@ EXPORTS = (
     "fsvd_exchange_region_bytes", "fsvd_exchange_region_alloc", "fsvd_exchange_region_free",
     "fsvd_exchange_region_export", "fsvd_exchange_region_import", "fsvd_exchange_region_release",
     "fsvd_exchange_create", "fsvd_exchange_destroy", "fsvd_exchange_set_trace", "fsvd_tp_workspace_bytes",
-    "fsvd_tp_decode_layer",
+    "fsvd_tp_decode_layer", "fsvd_prompt_create", "fsvd_prompt_run",
 )
 
 
@@ -98,6 +98,9 @@ def load() -> C.CDLL:
     lib.fsvd_model_create.argtypes = [
         C.POINTER(FsvdDims), C.POINTER(FsvdLayer), vp, vp, vp, vp, vp, ip, C.POINTER(vp)]
     lib.fsvd_model_destroy.argtypes = [vp]
+    lib.fsvd_prompt_create.argtypes = [
+        C.POINTER(FsvdDims), C.POINTER(FsvdLayer), vp, vp, vp, vp, vp, vp, C.POINTER(vp)]
+    lib.fsvd_prompt_run.argtypes = [vp, vp, ip, ip, vp]
     lib.fsvd_model_step.argtypes = [vp, ip, vp]
     lib.fsvd_model_buffers.argtypes = [vp] + [C.POINTER(vp)] * 6
     lib.fsvd_model_status.argtypes = [vp, C.POINTER(ip)]

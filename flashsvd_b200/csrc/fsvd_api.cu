@@ -1152,9 +1152,11 @@ struct fsvd_model {
   float* xbuf = nullptr;  // hidden state between layers, [B, d] of type T
   char* extra = nullptr;
   fsvd_tile_model* tile = nullptr;   // batches above 8: the tiled path owns everything
+  fsvd_tile_prompt* prompt = nullptr;   // prompt program of another model (fsvd_prompt_create)
 };
 
 int fsvd_model_destroy(fsvd_model* m);
+int fsvd_model_buffers(fsvd_model* m, int** tokens, int** seqlens, int** token_log, int** step_counter, float** logits, float** hidden);
 
 int fsvd_model_create(const fsvd_dims* dims, const fsvd_layer* layers, const void* embed,
                       const void* final_norm_w, const void* lm_head, const void* cos_tab,
@@ -1288,6 +1290,7 @@ int fsvd_model_create(const fsvd_dims* dims, const fsvd_layer* layers, const voi
 int fsvd_model_destroy(fsvd_model* m) {
   if (!m) return 0;
   if (m->tile) fsvd_tile_model_destroy(m->tile);
+  if (m->prompt) fsvd_tile_prompt_destroy(m->prompt);
   cudaFree(m->ws);
   cudaFree(m->extra);
   cudaFree(m->prog);
@@ -1299,6 +1302,7 @@ int fsvd_model_destroy(fsvd_model* m) {
 
 int fsvd_model_step(fsvd_model* m, int n_steps, void* stream) {
   if (!m) return fail(FSVD_ERR_ARG, "null model");
+  if (m->prompt) return fail(FSVD_ERR_ARG, "a prompt program takes prompts (fsvd_prompt_run), not steps");
   if (m->tile) return fsvd_tile_model_step(m->tile, n_steps, stream);
   SyncState* sync = reinterpret_cast<SyncState*>(m->ws + m->L.sync);
   const Settings set = current_settings();   // the geometry is the one of fsvd_model_create
@@ -1326,9 +1330,45 @@ int fsvd_model_step(fsvd_model* m, int n_steps, void* stream) {
   return 0;
 }
 
+// The dimensions of a prompt program: those of the decode model it fills the caches of.
+int fsvd_prompt_create(const fsvd_dims* dims, const fsvd_layer* layers, const void* embed, const void* final_norm_w,
+                       const void* lm_head, const void* cos_tab, const void* sin_tab, fsvd_model* decode, fsvd_model** out) {
+  if (!dims || !layers || !embed || !final_norm_w || !lm_head || !cos_tab || !sin_tab || !decode || !out)
+    return fail(FSVD_ERR_ARG, "null argument");
+  const fsvd_dims& D = *dims;
+  if (D.dtype != FSVD_DTYPE_BF16 || D.rows_are_positions) return fail(FSVD_ERR_UNSUPPORTED, "prompt programs need bf16 factors and one row per sequence");
+  if (decode->prompt || decode->D.B != D.B || decode->D.vocab != D.vocab || decode->D.S_max != D.S_max)
+    return fail(FSVD_ERR_ARG, "the decode model has another batch, vocabulary or cache length");
+  for (int l = 0; l < D.n_layers; ++l)
+    if (int e = check_layer_ptrs(layers[l])) return e;
+  if (!aligned16(embed) || !aligned16(lm_head) || !aligned16(final_norm_w) || !aligned16(cos_tab) || !aligned16(sin_tab))
+    return fail(FSVD_ERR_ALIGN, "embed / lm_head / norm / table pointers must be 16-byte aligned");
+  fsvd_tile_decode_state st;
+  memset(&st, 0, sizeof(st));
+  if (int e = fsvd_model_buffers(decode, &st.tokens, &st.seqlens, &st.token_log, &st.step_counter, &st.logits, nullptr)) return e;
+  st.max_steps = decode->max_steps < 1 ? 1 : decode->max_steps;
+  fsvd_tile_prompt* p = nullptr;
+  if (int e = fsvd_tile_prompt_create(dims, layers, embed, final_norm_w, lm_head, cos_tab, sin_tab, &st,
+                                      current_settings().wait_limit, &p))
+    return e;
+  fsvd_model* m = new fsvd_model();
+  m->D = D;
+  m->prompt = p;
+  *out = m;
+  return 0;
+}
+
+int fsvd_prompt_run(fsvd_model* m, const int* tokens, int row_stride, int length, void* stream) {
+  if (!m || !tokens) return fail(FSVD_ERR_ARG, "null argument");
+  if (!m->prompt) return fail(FSVD_ERR_ARG, "not a prompt program");
+  if (length < 1 || row_stride < length) return fail(FSVD_ERR_ARG, "prompt length %d with row stride %d", length, row_stride);
+  return fsvd_tile_prompt_run(m->prompt, tokens, row_stride, length, stream);
+}
+
 int fsvd_model_buffers(fsvd_model* m, int** tokens, int** seqlens, int** token_log,
                        int** step_counter, float** logits, float** hidden) {
   if (!m) return fail(FSVD_ERR_ARG, "null model");
+  if (m->prompt) return fail(FSVD_ERR_ARG, "a prompt program has no buffers of its own");
   if (m->tile) {
     fsvd_tile_model_buffers(m->tile, tokens, seqlens, token_log, step_counter, logits, hidden);
     return 0;
@@ -1342,16 +1382,18 @@ int fsvd_model_buffers(fsvd_model* m, int** tokens, int** seqlens, int** token_l
   return 0;
 }
 
-int fsvd_model_num_stages(fsvd_model* m) { return !m ? 0 : m->tile ? fsvd_tile_model_launches_per_step(m->tile) : m->nstages; }
-int fsvd_model_num_barriers(fsvd_model* m) { return (m && !m->tile) ? m->nbarriers : 0; }
+int fsvd_model_num_stages(fsvd_model* m) { return !m || m->prompt ? 0 : m->tile ? fsvd_tile_model_launches_per_step(m->tile) : m->nstages; }
+int fsvd_model_num_barriers(fsvd_model* m) { return (m && !m->tile && !m->prompt) ? m->nbarriers : 0; }
 
 int fsvd_model_status(fsvd_model* m, int* device_status) {
   if (!m) return fail(FSVD_ERR_ARG, "null model");
+  if (m->prompt) return fsvd_workspace_status(fsvd_tile_prompt_ws(m->prompt), device_status);
   return fsvd_workspace_status(m->tile ? fsvd_tile_model_ws(m->tile) : m->ws, device_status);
 }
 
 int fsvd_model_reset_sync(fsvd_model* m, void* stream) {
   if (!m) return fail(FSVD_ERR_ARG, "null model");
+  if (m->prompt) return fsvd_workspace_clear_status(fsvd_tile_prompt_ws(m->prompt), stream);
   if (m->tile) return fsvd_tile_model_reset(m->tile, stream);
   CUDA_TRY(cudaMemsetAsync(m->ws + m->L.sync, 0, sizeof(SyncState), (cudaStream_t)stream));
   CUDA_TRY(cudaMemsetAsync(m->ws + m->L.counters, 0, kCounterBytes, (cudaStream_t)stream));

@@ -22,7 +22,8 @@
 // factors with the q / k / v lifts grouped, attention with the split merge inside the kernel); a
 // model step is captured once into a CUDA graph.  Attention: batch_attn_kernel (1 or 2 query heads per
 // kv head, shuffle-reduced dot products at the HBM rate), gqa_decode_attn_kernel (4 or 8: the heads as
-// rows of a tensor-core tile), prompt_attn_kernel (causal attention of a prompt pass).
+// rows of a tensor-core tile).  The prompt pass (whole prompts as rows, fsvd_prompt_run) has its GEMM and
+// attention kernels in fsvd_prompt.cuh.
 // Tensor-parallel layer (fsvd_tile_tp_decode_layer): the o lift and the down lift end in the push
 // epilogue (TE_PUSH: partial sums stored into every rank's exchange region over peer memory, one flag
 // per CTA), exchange_reduce_rows_kernel sums them in rank order with the residual and applies the
@@ -43,6 +44,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <initializer_list>
 #include <mutex>
 #include <utility>
 #include <vector>
@@ -50,18 +52,11 @@
 #include "../../include/flashsvd_b200.h"
 #include "fsvd_exchange.h"
 #include "fsvd_stage.h"
+#include "fsvd_tc.cuh"
 #include "fsvd_tile.h"
 
 namespace fsvd_tile {
 
-using fsvd::DS_BARRIER_TIMEOUT;
-using fsvd::DS_CACHE_FULL;
-using fsvd::DS_COPY_TIMEOUT;
-using fsvd::DS_OK;
-using fsvd::SyncState;
-
-constexpr int kTileM = 128;          // factor rows of a tile (UMMA M)
-constexpr int kTileK = 64;           // bf16 elements of a k-block: one 128-byte swizzle span
 constexpr int kThreads = 128;        // 4 warps: warp w reads accumulator lanes 32 w .. 32 w + 31
 constexpr int kWTileBytes = kTileM * kTileK * 2;   // 16 KB
 constexpr int kMaxStages = 8;
@@ -99,88 +94,6 @@ struct GemmArgs {
   const unsigned* ex_seq;      // TE_PUSH: this rank's exchange sequence number
 };
 
-// ------------------------------------------------------------------------------- PTX
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-__device__ __forceinline__ void tma_box_2d(uint32_t dst, const void* tmap, int col, int row, uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-      ::"r"(dst), "l"(tmap), "r"(col), "r"(row), "r"(bar)
-      : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_alloc(uint32_t slot, uint32_t cols) {
-  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot), "r"(cols) : "memory");
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tc_dealloc(uint32_t taddr, uint32_t cols) {
-  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
-}
-// D[tmem] (+)= A[smem] . B[smem]^T, one 128 x N x 16 step
-__device__ __forceinline__ void tc_mma(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// the mbarrier gets one arrival when every MMA issued so far by this thread has finished
-__device__ __forceinline__ void tc_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-// 16 consecutive accumulator columns of this thread's lane
-__device__ __forceinline__ void tc_ld16(uint32_t taddr, float (&v)[16]) {
-  uint32_t r[16];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr)
-      : "memory");
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
-}
-
-// Shared-memory operand descriptor: K-major tile of rows x 64 bf16, 128-byte swizzle (the layout a
-// TMA box of 64 columns with CU_TENSOR_MAP_SWIZZLE_128B leaves): 8-row groups are 1024 bytes apart.
-__device__ __forceinline__ uint64_t umma_desc(uint32_t smem_addr) {
-  return (uint64_t)((smem_addr >> 4) & 0x3FFFu) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
-}
-// Instruction descriptor: bf16 x bf16 -> fp32, both operands K-major, M = 128, N.
-__device__ __forceinline__ uint32_t umma_idesc(int N) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(kTileM >> 4) << 24);
-}
-
-// Cluster barrier (all threads of all CTAs of the cluster) and a store into the shared memory of
-// the cluster's CTA `rank` at the same offset as the local address `addr`.
-__device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void st_cluster_v4(uint32_t addr, uint32_t rank, float x, float y, float z, float w) {
-  uint32_t remote;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
-  asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(remote), "f"(x), "f"(y), "f"(z), "f"(w) : "memory");
-}
-
 __device__ __forceinline__ void tmark(const GemmArgs& a, int k) {
   if (a.trace && threadIdx.x == 0) {
     unsigned long long t;
@@ -188,40 +101,6 @@ __device__ __forceinline__ void tmark(const GemmArgs& a, int k) {
     a.trace[((size_t)(blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) * 16 + k] = t;
   }
 }
-
-__device__ __forceinline__ float rnd(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
-__device__ __forceinline__ float ldbf(const void* p, size_t i) {
-  return __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p)[i]);
-}
-__device__ __forceinline__ void stbf(void* p, size_t i, float v) {
-  reinterpret_cast<__nv_bfloat16*>(p)[i] = __float2bfloat16_rn(v);
-}
-
-// Bounded mbarrier wait; false when the budget ran out or the CTA has given up already.
-__device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, volatile int* giveup, const GemmArgs& a, int code) {
-  if (mbar_try_wait(bar, parity)) return true;
-  if (*giveup) return false;
-  const long long c0 = clock64();
-  unsigned spins = 0;
-  while (!mbar_try_wait(bar, parity)) {
-    if ((++spins & 63u) == 0) {
-      if (*giveup) return false;
-      if (clock64() - c0 > a.wait_limit) {
-        atomicCAS(a.status, (int)DS_OK, code);
-        *giveup = 1;
-        return false;
-      }
-    }
-  }
-  return true;
-}
-
-// Programmatic dependent launch: every kernel of this file is launched with the stream-serialization
-// attribute, so its CTAs may start while the kernel before it in the stream is still draining.
-// pdl_wait() returns when that kernel has completed and its writes are visible; nothing that
-// another kernel wrote is read, and nothing in global memory is written, before it.
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // Up to three independent GEMMs in one launch (the q, k and v lifts of a layer): blockIdx.z picks
 // the problem, CTAs outside a problem's (tiles, segs) range leave at once.
@@ -305,7 +184,7 @@ __global__ void __launch_bounds__(kThreads) tile_gemm_kernel(const __grid_consta
       for (int it = 0; it < nit; ++it) {
         const int s = it % NS, round = it / NS;
         if (s % kProducers != pj) continue;
-        if (round > 0 && !wait_bar(empty0 + 8 * s, (uint32_t)(round - 1) & 1u, giveup, a, DS_COPY_TIMEOUT)) break;
+        if (round > 0 && !wait_bar(empty0 + 8 * s, (uint32_t)(round - 1) & 1u, giveup, a.status, a.wait_limit, DS_COPY_TIMEOUT)) break;
         const uint32_t fb = full0 + 8 * s;
         uint32_t dst = base + (uint32_t)s * stage_bytes;
         const int kcol = (kb0 + it) * kTileK;
@@ -329,7 +208,7 @@ __global__ void __launch_bounds__(kThreads) tile_gemm_kernel(const __grid_consta
       pdl_wait();
       for (int it = 0; it < nit && ok; ++it) {
         const int s = it % NS, round = it / NS;
-        ok = wait_bar(full0 + 8 * s, (uint32_t)round & 1u, giveup, a, DS_COPY_TIMEOUT);
+        ok = wait_bar(full0 + 8 * s, (uint32_t)round & 1u, giveup, a.status, a.wait_limit, DS_COPY_TIMEOUT);
         if (!ok) break;
         tc_fence_after();
         const uint32_t sa = base + (uint32_t)s * stage_bytes;
@@ -367,7 +246,7 @@ __global__ void __launch_bounds__(kThreads) tile_gemm_kernel(const __grid_consta
           asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const __nv_bfloat16*>(a.resid) + (size_t)b * a.P + prow));
       }
   }
-  bool have = nit > 0 ? wait_bar(accum, 0u, giveup, a, DS_BARRIER_TIMEOUT) : false;
+  bool have = nit > 0 ? wait_bar(accum, 0u, giveup, a.status, a.wait_limit, DS_BARRIER_TIMEOUT) : false;
   have = __all_sync(0xffffffffu, have);
   tc_fence_after();
   tmark(a, 3);
@@ -526,19 +405,41 @@ __global__ void __launch_bounds__(kThreads) tile_gemm_kernel(const __grid_consta
 }
 
 // ------------------------------------------------------------------------------- RMSNorm rows
-// out[b, :] = rnd(w * rnd(x[b, :] * rsqrt(mean(x[b, :]^2) + eps))), one CTA per row.
+// out[b, :] = rnd(w * rnd(x[r, :] * rsqrt(mean(x[r, :]^2) + eps))), r = b * row_mul + row_off, one CTA per
+// row.  A thread's 16-byte pieces stay in registers between the two passes (rows up to 8192 wide).
 __global__ void __launch_bounds__(256) rmsnorm_rows_kernel(const __nv_bfloat16* __restrict__ x,
                                                            const __nv_bfloat16* __restrict__ w,
-                                                           __nv_bfloat16* __restrict__ out, int d, float eps) {
+                                                           __nv_bfloat16* __restrict__ out, int d, float eps,
+                                                           int row_mul, int row_off) {
+  constexpr int U = 4;
   __shared__ float red[8];
-  const int b = blockIdx.x, tid = threadIdx.x;
+  const int b = blockIdx.x, tid = threadIdx.x, n8 = d >> 3;
   pdl_launch_dependents();
   pdl_wait();
-  const __nv_bfloat16* xr = x + (size_t)b * d;
+  const uint4* xr = reinterpret_cast<const uint4*>(x + (size_t)(b * row_mul + row_off) * d);
+  const uint4* wr = reinterpret_cast<const uint4*>(w);
+  uint4* orow = reinterpret_cast<uint4*>(out + (size_t)b * d);
+  const bool fits = n8 <= 256 * U;
+  uint4 v[U], wv[U];
   float ss = 0.0f;
-  for (int i = tid; i < d; i += 256) {
-    const float v = __bfloat162float(xr[i]);
-    ss += v * v;
+  for (int i0 = tid; i0 < n8; i0 += 256 * U) {
+#pragma unroll
+    for (int k = 0; k < U; ++k)
+      if (i0 + 256 * k < n8) {
+        v[k] = xr[i0 + 256 * k];
+        wv[k] = wr[i0 + 256 * k];
+      }
+#pragma unroll
+    for (int k = 0; k < U; ++k)
+      if (i0 + 256 * k < n8) {
+        const uint32_t u[4] = {v[k].x, v[k].y, v[k].z, v[k].w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float lo = __uint_as_float(u[j] << 16), hi = __uint_as_float(u[j] & 0xffff0000u);
+          ss += lo * lo;
+          ss += hi * hi;
+        }
+      }
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
@@ -548,8 +449,22 @@ __global__ void __launch_bounds__(256) rmsnorm_rows_kernel(const __nv_bfloat16* 
 #pragma unroll
   for (int i = 0; i < 8; ++i) tot += red[i];
   const float inv = rsqrtf(tot / (float)d + eps);
-  for (int i = tid; i < d; i += 256)
-    out[(size_t)b * d + i] = __float2bfloat16_rn(__bfloat162float(w[i]) * rnd(__bfloat162float(xr[i]) * inv));
+  auto finish = [&](int i, const uint4& xq, const uint4& wq) {
+    const uint32_t xu[4] = {xq.x, xq.y, xq.z, xq.w}, wu[4] = {wq.x, wq.y, wq.z, wq.w};
+    uint32_t o[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      o[j] = pack_bf16(__uint_as_float(wu[j] << 16) * rnd(__uint_as_float(xu[j] << 16) * inv),
+                       __uint_as_float(wu[j] & 0xffff0000u) * rnd(__uint_as_float(xu[j] & 0xffff0000u) * inv));
+    orow[i] = make_uint4(o[0], o[1], o[2], o[3]);
+  };
+  if (fits) {
+#pragma unroll
+    for (int k = 0; k < U; ++k)
+      if (tid + 256 * k < n8) finish(tid + 256 * k, v[k], wv[k]);
+  } else {
+    for (int i = tid; i < n8; i += 256) finish(i, xr[i], wr[i]);
+  }
 }
 
 // ------------------------------------------------------------------------------- exchange + RMSNorm rows
@@ -740,15 +655,11 @@ __device__ __forceinline__ void ld_row<2>(const __nv_bfloat16* row, int lane, fl
   f[0] = __uint_as_float(w << 16); f[1] = __uint_as_float(w & 0xffff0000u);
 }
 
-// RB > 1 (prompt pass: the batch rows are consecutive positions of one sequence and share its cache):
-// a CTA takes RB consecutive rows of one kv head, so a key / value row is read once for RB x G
-// query vectors; every (row, head) slot has its own causal limit.  RB > 1 runs with one split.
-template <int DH, int G, int RB>
+template <int DH, int G>
 __global__ void __launch_bounds__(kAttnThreads) batch_attn_kernel(const AttnArgs a) {
   constexpr int DPL = DH / 32;
-  constexpr int NG = G * RB;                     // query vectors that share the rows this CTA reads
-  __shared__ float wm[kAttnWarps][NG], wl[kAttnWarps][NG];
-  __shared__ float wacc[kAttnWarps][NG][DH];
+  __shared__ float wm[kAttnWarps][G], wl[kAttnWarps][G];
+  __shared__ float wacc[kAttnWarps][G][DH];
   __shared__ int last_sh;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   pdl_launch_dependents();
@@ -756,28 +667,19 @@ __global__ void __launch_bounds__(kAttnThreads) batch_attn_kernel(const AttnArgs
   int idx = blockIdx.x;
   const int split = idx % a.nsplit;
   idx /= a.nsplit;
-  const int hk = idx % a.Hk, b = idx / a.Hk;     // b: batch row, or block of RB rows
-  const int row0 = b * RB;
-  int nl[RB];                                    // keys visible to each of the CTA's rows
-  int n = 0;
-#pragma unroll
-  for (int r = 0; r < RB; ++r) {
-    const int row = row0 + r;
-    nl[r] = row < a.B ? min(a.seqlens[row] + a.seqlen_add, a.S_max) : 0;
-    n = max(n, nl[r]);
-  }
+  const int hk = idx % a.Hk, b = idx / a.Hk;
+  const int n = min(a.seqlens[b] + a.seqlen_add, a.S_max);
   const int per = (n + a.nsplit - 1) / a.nsplit;
   const int j0 = min(n, split * per), j1 = min(n, j0 + per);
   const size_t rowstride = (size_t)a.Hk * DH;
-  const size_t cbase = ((size_t)(a.shared_cache ? 0 : row0) * a.S_max) * rowstride + (size_t)hk * DH;
+  const size_t cbase = ((size_t)b * a.S_max) * rowstride + (size_t)hk * DH;
   const __nv_bfloat16* kbase = a.kcache + cbase;
   const __nv_bfloat16* vbase = a.vcache + cbase;
 
-  float q[NG][DPL], acc[NG][DPL], m[NG], l[NG];
+  float q[G][DPL], acc[G][DPL], m[G], l[G];
 #pragma unroll
-  for (int g = 0; g < NG; ++g) {
-    const int row = min(row0 + g / G, a.B - 1);
-    ld_row<DPL>(a.q + ((size_t)row * a.H + hk * G + g % G) * DH, lane, q[g]);
+  for (int g = 0; g < G; ++g) {
+    ld_row<DPL>(a.q + ((size_t)b * a.H + hk * G + g) * DH, lane, q[g]);
 #pragma unroll
     for (int e = 0; e < DPL; ++e) {
       q[g][e] *= a.scale;
@@ -797,7 +699,7 @@ __global__ void __launch_bounds__(kAttnThreads) batch_attn_kernel(const AttnArgs
       ld_row<DPL>(vbase + (size_t)row * rowstride, lane, vf[i]);
     }
 #pragma unroll
-    for (int g = 0; g < NG; ++g) {
+    for (int g = 0; g < G; ++g) {
       float s[kKeyGroup];
 #pragma unroll
       for (int i = 0; i < kKeyGroup; ++i) {
@@ -815,20 +717,17 @@ __global__ void __launch_bounds__(kAttnThreads) batch_attn_kernel(const AttnArgs
 #pragma unroll
       for (int i = 0; i < kKeyGroup; ++i) {
         if (i >= cn) s[i] = -INFINITY;                          // past the split
-        if (RB > 1 && c0 + i >= nl[g / G]) s[i] = -INFINITY;    // past this query's position
         cm = fmaxf(cm, s[i]);
       }
       const float mn = fmaxf(m[g], cm);
-      // (with row blocks a whole group can be invisible to an early row: every weight below is then 0)
-      const float mref = (RB > 1 && mn == -INFINITY) ? 0.0f : mn;
-      const float corr = __expf(m[g] - mref);               // 0 when m is still -inf
+      const float corr = __expf(m[g] - mn);                 // 0 when m is still -inf
       m[g] = mn;
       float ps = 0.0f;
 #pragma unroll
       for (int e = 0; e < DPL; ++e) acc[g][e] *= corr;
 #pragma unroll
       for (int i = 0; i < kKeyGroup; ++i) {
-        const float pr = __expf(s[i] - mref);               // 0 for the masked rows
+        const float pr = __expf(s[i] - mn);               // 0 for the masked rows
         ps += pr;
 #pragma unroll
         for (int e = 0; e < DPL; ++e) acc[g][e] += pr * vf[i][e];
@@ -838,7 +737,7 @@ __global__ void __launch_bounds__(kAttnThreads) batch_attn_kernel(const AttnArgs
   }
   // ---- the warps meet
 #pragma unroll
-  for (int g = 0; g < NG; ++g) {
+  for (int g = 0; g < G; ++g) {
     if (lane == 0) {
       wm[warp][g] = m[g];
       wl[warp][g] = l[g];
@@ -849,10 +748,9 @@ __global__ void __launch_bounds__(kAttnThreads) batch_attn_kernel(const AttnArgs
   __syncthreads();
   const int nsplit = a.nsplit;
   const int rec = DH + 2;
-  float* mine = a.part + ((((size_t)b * a.Hk + hk) * nsplit + split) * NG) * rec;
-  for (int i = tid; i < NG * DH; i += kAttnThreads) {
+  float* mine = a.part + ((((size_t)b * a.Hk + hk) * nsplit + split) * G) * rec;
+  for (int i = tid; i < G * DH; i += kAttnThreads) {
     const int g = i / DH, dd = i - g * DH;
-    const int row = row0 + g / G;
     float mm = -INFINITY;
 #pragma unroll
     for (int w = 0; w < kAttnWarps; ++w) mm = fmaxf(mm, wm[w][g]);
@@ -864,8 +762,7 @@ __global__ void __launch_bounds__(kAttnThreads) batch_attn_kernel(const AttnArgs
       den += wgt * wl[w][g];
     }
     if (nsplit == 1) {
-      if (row < a.B)
-        a.out[((size_t)row * a.H + hk * G + g % G) * DH + dd] = __float2bfloat16_rn(den > 0.0f ? num / den : 0.0f);
+      a.out[((size_t)b * a.H + hk * G + g) * DH + dd] = __float2bfloat16_rn(den > 0.0f ? num / den : 0.0f);
     } else {
       mine[(size_t)g * rec + dd] = num;
       if (dd == 0) {
@@ -885,195 +782,20 @@ __global__ void __launch_bounds__(kAttnThreads) batch_attn_kernel(const AttnArgs
   __syncthreads();
   if (!last_sh) return;
   __threadfence();
-  const float* parts = a.part + (((size_t)b * a.Hk + hk) * nsplit) * NG * rec;
-  for (int i = tid; i < NG * DH; i += kAttnThreads) {
+  const float* parts = a.part + (((size_t)b * a.Hk + hk) * nsplit) * G * rec;
+  for (int i = tid; i < G * DH; i += kAttnThreads) {
     const int g = i / DH, dd = i - g * DH;
-    const int row = row0 + g / G;
     float mm = -INFINITY;
-    for (int sp = 0; sp < nsplit; ++sp) mm = fmaxf(mm, __ldcg(parts + ((size_t)sp * NG + g) * rec + DH));
+    for (int sp = 0; sp < nsplit; ++sp) mm = fmaxf(mm, __ldcg(parts + ((size_t)sp * G + g) * rec + DH));
     float num = 0.0f, den = 0.0f;
     for (int sp = 0; sp < nsplit; ++sp) {
-      const float* pr = parts + ((size_t)sp * NG + g) * rec;
+      const float* pr = parts + ((size_t)sp * G + g) * rec;
       const float ms = __ldcg(pr + DH);
       const float wgt = ms == -INFINITY ? 0.0f : __expf(ms - mm);
       num += wgt * __ldcg(pr + dd);
       den += wgt * __ldcg(pr + DH + 1);
     }
-    if (row < a.B)
-      a.out[((size_t)row * a.H + hk * G + g % G) * DH + dd] = __float2bfloat16_rn(den > 0.0f ? num / den : 0.0f);
-  }
-}
-
-// ------------------------------------------------------------------------------- prompt-pass attention
-// Causal attention of a block of consecutive prompt rows over the one sequence's cache, on the
-// tensor cores (mma.sync m16n8k16 / bf16, fp32 accumulation): the rows of a pass share the cache
-// rows they read, so a key / value block staged in shared memory serves 32 query vectors
-// (32 / G rows x G heads of one kv head, 16 per warp).  Per block of 64 keys: S = Q K^T (the key rows
-// are the col-major B operand as they lie), causal mask by absolute position, running softmax,
-// O += P V with the value fragments taken through ldmatrix.trans.  Replaces the row-block variant
-// of batch_attn_kernel for the prompt pass (the reference: kernels/attn/prefill/rope_sdpa.py:67-427).
-constexpr int kPfWarps = 2;
-constexpr int kPfSlots = 16 * kPfWarps;     // query vectors per CTA
-constexpr int kPfKeys = 64;                 // keys per block
-
-__device__ __forceinline__ void mma_bf16_16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
-                                               uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
-  const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
-  return *reinterpret_cast<const uint32_t*>(&v);
-}
-
-template <int DH>
-__global__ void __launch_bounds__(kPfWarps * 32) prompt_attn_kernel(const AttnArgs a) {
-  constexpr int STRIDE = DH * 2 + 16;                 // bytes of a staged row (16 bytes of padding: no bank conflicts)
-  constexpr int KS = DH / 16;                         // k-steps of Q K^T
-  constexpr int NT = kPfKeys / 8;                     // score tiles per key block
-  constexpr int DT = DH / 8;                          // output tiles
-  __shared__ __align__(16) unsigned char ks_s[kPfKeys * STRIDE];
-  __shared__ __align__(16) unsigned char vs_s[kPfKeys * STRIDE];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-  pdl_launch_dependents();
-  pdl_wait();
-  const int G = a.H / a.Hk;
-  const int rpb = kPfSlots / G;                       // rows per CTA
-  const int hk = blockIdx.y, row0 = blockIdx.x * rpb;
-  // this thread's two query vectors: slots m0 and m0 + 8 of the CTA
-  const int m0 = warp * 16 + g;
-  int rowq[2], headq[2], nl[2];
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const int m = m0 + 8 * i;
-    rowq[i] = row0 + m / G;
-    headq[i] = hk * G + m % G;
-    nl[i] = rowq[i] < a.B ? min(a.seqlens[rowq[i]] + a.seqlen_add, a.S_max) : 0;
-  }
-  const int last_row = min(row0 + rpb, a.B) - 1;
-  const int nmax = last_row >= row0 ? min(a.seqlens[last_row] + a.seqlen_add, a.S_max) : 0;   // positions increase with the row
-  // Q fragments (rows g and g + 8 of the warp's 16, dims 16 ks + 2 t .. and + 8)
-  uint32_t qa[KS][4];
-#pragma unroll
-  for (int ks = 0; ks < KS; ++ks) {
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const __nv_bfloat16* qp = a.q + ((size_t)min(rowq[i], a.B - 1) * a.H + headq[i]) * DH + ks * 16 + 2 * t;
-      qa[ks][i] = *reinterpret_cast<const uint32_t*>(qp);
-      qa[ks][2 + i] = *reinterpret_cast<const uint32_t*>(qp + 8);
-    }
-  }
-  float o[DT][4];
-#pragma unroll
-  for (int d = 0; d < DT; ++d) o[d][0] = o[d][1] = o[d][2] = o[d][3] = 0.0f;
-  float mrow[2] = {-INFINITY, -INFINITY}, lrow[2] = {0.0f, 0.0f};
-  const size_t rowstride = (size_t)a.Hk * DH;
-  const __nv_bfloat16* kbase = a.kcache + (size_t)hk * DH;     // shared cache: row 0 of the cache tensor
-  const __nv_bfloat16* vbase = a.vcache + (size_t)hk * DH;
-
-  for (int k0 = 0; k0 < nmax; k0 += kPfKeys) {
-    // ---- stage 64 key rows and 64 value rows (zeros past the visible range)
-    __syncthreads();
-    for (int i = tid; i < kPfKeys * (DH / 8); i += kPfWarps * 32) {
-      const int r = i / (DH / 8), c = i - r * (DH / 8);
-      uint4 kv = make_uint4(0, 0, 0, 0), vv = kv;
-      if (k0 + r < nmax) {
-        kv = __ldg(reinterpret_cast<const uint4*>(kbase + (size_t)(k0 + r) * rowstride) + c);
-        vv = __ldg(reinterpret_cast<const uint4*>(vbase + (size_t)(k0 + r) * rowstride) + c);
-      }
-      *reinterpret_cast<uint4*>(ks_s + r * STRIDE + c * 16) = kv;
-      *reinterpret_cast<uint4*>(vs_s + r * STRIDE + c * 16) = vv;
-    }
-    __syncthreads();
-    // ---- S = Q K^T for this warp's 16 query vectors x 64 keys
-    float sc[NT][4];
-#pragma unroll
-    for (int nt = 0; nt < NT; ++nt) {
-      sc[nt][0] = sc[nt][1] = sc[nt][2] = sc[nt][3] = 0.0f;
-      const unsigned char* kr = ks_s + (nt * 8 + g) * STRIDE + 4 * t;
-#pragma unroll
-      for (int ks = 0; ks < KS; ++ks) {
-        const uint32_t b0 = *reinterpret_cast<const uint32_t*>(kr + ks * 32);
-        const uint32_t b1 = *reinterpret_cast<const uint32_t*>(kr + ks * 32 + 16);
-        mma_bf16_16816(sc[nt], qa[ks][0], qa[ks][1], qa[ks][2], qa[ks][3], b0, b1);
-      }
-    }
-    // ---- scale, causal mask, running softmax (rows g and g + 8; a row's 64 scores sit in 4 lanes)
-    float mx[2] = {-INFINITY, -INFINITY};
-#pragma unroll
-    for (int nt = 0; nt < NT; ++nt) {
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int i = e >> 1;
-        const int kj = k0 + nt * 8 + 2 * t + (e & 1);
-        const float v = kj < nl[i] ? sc[nt][e] * a.scale : -INFINITY;
-        sc[nt][e] = v;
-        mx[i] = fmaxf(mx[i], v);
-      }
-    }
-    float corr[2], mref[2];
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      mx[i] = fmaxf(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], 1));
-      mx[i] = fmaxf(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], 2));
-      const float mn = fmaxf(mrow[i], mx[i]);
-      mref[i] = mn == -INFINITY ? 0.0f : mn;          // nothing visible yet: every weight is 0
-      corr[i] = __expf(mrow[i] - mref[i]);
-      mrow[i] = mn;
-    }
-    float ps[2] = {0.0f, 0.0f};
-#pragma unroll
-    for (int nt = 0; nt < NT; ++nt) {
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float pr = __expf(sc[nt][e] - mref[e >> 1]);
-        sc[nt][e] = pr;
-        ps[e >> 1] += pr;
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      ps[i] += __shfl_xor_sync(0xffffffffu, ps[i], 1);
-      ps[i] += __shfl_xor_sync(0xffffffffu, ps[i], 2);
-      lrow[i] = lrow[i] * corr[i] + ps[i];
-    }
-#pragma unroll
-    for (int d = 0; d < DT; ++d) {
-      o[d][0] *= corr[0]; o[d][1] *= corr[0];
-      o[d][2] *= corr[1]; o[d][3] *= corr[1];
-    }
-    // ---- O += P V: 16 keys per step; the P fragments are the score tiles as they lie
-#pragma unroll
-    for (int kk = 0; kk < kPfKeys / 16; ++kk) {
-      const uint32_t pa0 = pack_bf16(sc[2 * kk][0], sc[2 * kk][1]);
-      const uint32_t pa1 = pack_bf16(sc[2 * kk][2], sc[2 * kk][3]);
-      const uint32_t pa2 = pack_bf16(sc[2 * kk + 1][0], sc[2 * kk + 1][1]);
-      const uint32_t pa3 = pack_bf16(sc[2 * kk + 1][2], sc[2 * kk + 1][3]);
-      // ldmatrix.x4.trans: matrices (keys 16 kk .. + 7, dims 16 j .. + 7), (keys + 8, same dims),
-      // (keys .. + 7, dims + 8), (keys + 8, dims + 8) -> b0, b1 of output tile 2 j and of tile 2 j + 1
-      const int lrow_ = kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8;
-      const unsigned char* vr = vs_s + lrow_ * STRIDE + ((lane >> 4) & 1) * 16;
-#pragma unroll
-      for (int j = 0; j < DT / 2; ++j) {
-        uint32_t b0, b1, b2, b3;
-        const uint32_t addr = (uint32_t)__cvta_generic_to_shared(vr + j * 32);
-        asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-                     : "=r"(b0), "=r"(b1), "=r"(b2), "=r"(b3) : "r"(addr));
-        mma_bf16_16816(o[2 * j], pa0, pa1, pa2, pa3, b0, b1);
-        mma_bf16_16816(o[2 * j + 1], pa0, pa1, pa2, pa3, b2, b3);
-      }
-    }
-  }
-  // ---- normalise and store: thread holds (row g, dims 8 d + 2 t, + 1) and (row g + 8, same dims)
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    if (rowq[i] >= a.B) continue;
-    const float inv = lrow[i] > 0.0f ? 1.0f / lrow[i] : 0.0f;
-    __nv_bfloat16* op = a.out + ((size_t)rowq[i] * a.H + headq[i]) * DH + 2 * t;
-#pragma unroll
-    for (int d = 0; d < DT; ++d)
-      *reinterpret_cast<uint32_t*>(op + d * 8) = pack_bf16(o[d][2 * i] * inv, o[d][2 * i + 1] * inv);
+    a.out[((size_t)b * a.H + hk * G + g) * DH + dd] = __float2bfloat16_rn(den > 0.0f ? num / den : 0.0f);
   }
 }
 
@@ -1108,7 +830,7 @@ __global__ void __launch_bounds__(kAttnThreads, 3) gqa_decode_attn_kernel(const 
   const int per = ((n + a.nsplit - 1) / a.nsplit + kGqKeys - 1) / kGqKeys * kGqKeys;   // whole blocks per split
   const int j0 = min(n, split * per), j1 = min(n, j0 + per);
   const size_t rowstride = (size_t)a.Hk * DH;
-  const size_t cbase = ((size_t)(a.shared_cache ? 0 : b) * a.S_max) * rowstride + (size_t)hk * DH;
+  const size_t cbase = ((size_t)b * a.S_max) * rowstride + (size_t)hk * DH;
   const __nv_bfloat16* kbase = a.kcache + cbase;
   const __nv_bfloat16* vbase = a.vcache + cbase;
   unsigned char* ks_s = gq_smem + (size_t)warp * (2 * kGqKeys * STRIDE);
@@ -1314,22 +1036,49 @@ __global__ void __launch_bounds__(kAttnThreads, 3) gqa_decode_attn_kernel(const 
   }
 }
 
+}  // namespace fsvd_tile
+#include "fsvd_prompt.cuh"
+namespace fsvd_tile {
+
 // ------------------------------------------------------------------------------- step head / tail
+__device__ __forceinline__ void copy_row(const __nv_bfloat16* __restrict__ src, __nv_bfloat16* __restrict__ dst, int d) {
+  for (int i = threadIdx.x; i < (d >> 3); i += blockDim.x) reinterpret_cast<uint4*>(dst)[i] = reinterpret_cast<const uint4*>(src)[i];
+}
 __global__ void embed_rows_kernel(const __nv_bfloat16* __restrict__ table, const int* __restrict__ tokens,
                                   __nv_bfloat16* __restrict__ out, int d, int vocab) {
   const int b = blockIdx.x;
   pdl_launch_dependents();
   pdl_wait();
-  int tok = tokens[b];
-  tok = min(max(tok, 0), vocab - 1);
-  for (int i = threadIdx.x; i < d; i += blockDim.x) out[(size_t)b * d + i] = table[(size_t)tok * d + i];
+  const int tok = min(max(tokens[b], 0), vocab - 1);
+  copy_row(table + (size_t)tok * d, out + (size_t)b * d, d);
+}
+// First kernel of a prompt pass: row r = b n + t takes token prompt[b, off + t] at position
+// seqlens[b] + t of sequence b.
+__global__ void prompt_begin_kernel(const __nv_bfloat16* __restrict__ table, const int* __restrict__ prompt, int ld, int off, int n,
+                                    const int* __restrict__ seqlens, int* rowpos, int* rowseq, __nv_bfloat16* __restrict__ out,
+                                    int d, int vocab) {
+  const int r = blockIdx.x, b = r / n, t = r - b * n;
+  pdl_launch_dependents();
+  pdl_wait();
+  if (threadIdx.x == 0) {
+    rowpos[r] = seqlens[b] + t;
+    rowseq[r] = b;
+  }
+  const int tok = min(max(prompt[(size_t)b * ld + off + t], 0), vocab - 1);
+  copy_row(table + (size_t)tok * d, out + (size_t)r * d, d);
+}
+// Last kernel of a prompt pass that is not the prompt's last.
+__global__ void advance_kernel(int* seqlens, int nseq, int n) {
+  pdl_launch_dependents();
+  pdl_wait();
+  if ((int)threadIdx.x < nseq) seqlens[threadIdx.x] += n;
 }
 
 // token[b] = argmax_v logits[b, v] (lowest index among equal maxima); logs it; CTA 0 of the last
 // row... every row advances its own sequence length, row 0 the step counter.
 __global__ void __launch_bounds__(256) argmax_rows_kernel(const float* __restrict__ logits, int vocab, int* tokens,
                                                           int* token_log, int* step_counter, int* seqlens,
-                                                          int max_steps, int B) {
+                                                          int max_steps, int B, int advance) {
   __shared__ float bv[8];
   __shared__ int bi[8];
   const int b = blockIdx.x, tid = threadIdx.x;
@@ -1369,7 +1118,7 @@ __global__ void __launch_bounds__(256) argmax_rows_kernel(const float* __restric
     tokens[b] = besti;
     const int step = *step_counter;
     if (token_log && step < max_steps) token_log[(size_t)step * B + b] = besti;
-    seqlens[b] += 1;
+    seqlens[b] += advance;
   }
 }
 __global__ void bump_step_kernel(int* step_counter) {
@@ -1755,30 +1504,32 @@ static int plan_layer(LayerPlan& lp, const fsvd_dims& D, const fsvd_layer& Lw, c
 }
 
 template <int DH>
+static void launch_prompt_attn(const PaArgs& pa, int nseq, cudaStream_t st) {
+  constexpr int smem = 4 * kPaKeys * (DH * 2 + 16);
+  static bool attr_set = false;   // per instantiation; set under the planner's lock or at first use
+  if (!attr_set) {
+    cudaFuncSetAttribute(prompt_attn_kernel<DH>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    attr_set = true;
+  }
+  const int rpb = kPaSlots / (pa.H / pa.Hk);
+  launch_pdl(prompt_attn_kernel<DH>, dim3((unsigned)((pa.L + rpb - 1) / rpb), (unsigned)pa.Hk, (unsigned)nseq), dim3(kPaWarps * 32),
+             (size_t)smem, st, pa);
+}
+// rows of nseq sequences, L consecutive positions each
+static void launch_prompt_attn(const PaArgs& pa, int Dh, int nseq, cudaStream_t st) {
+  if (Dh == 128) launch_prompt_attn<128>(pa, nseq, st);
+  else launch_prompt_attn<64>(pa, nseq, st);
+  fsvd_tile_count_launch();
+}
+
+template <int DH>
 static void launch_attn_g(const AttnArgs& at, cudaStream_t st) {
   const unsigned threads = kAttnThreads;
   const int G = at.H / at.Hk;
-  if (at.shared_cache && at.nsplit == 1 && at.B >= 16) {
-    // prompt pass: tensor-core attention, 32 / G rows of one kv head per CTA
-    const int rpb = kPfSlots / G;
-    launch_pdl(prompt_attn_kernel<DH>, dim3((unsigned)((at.B + rpb - 1) / rpb), (unsigned)at.Hk), dim3(kPfWarps * 32), 0, st, at);
-    return;
-  }
-  if (at.shared_cache && at.nsplit == 1 && G < 8) {
-    // prompt pass: blocks of 8 / G consecutive rows share the key and value rows they read
-    const int RB = 8 / G;
-    const unsigned grid = (unsigned)(((at.B + RB - 1) / RB) * at.Hk);
-    switch (G) {
-      case 1: launch_pdl(batch_attn_kernel<DH, 1, 8>, dim3(grid), dim3(threads), 0, st, at); break;
-      case 2: launch_pdl(batch_attn_kernel<DH, 2, 4>, dim3(grid), dim3(threads), 0, st, at); break;
-      default: launch_pdl(batch_attn_kernel<DH, 4, 2>, dim3(grid), dim3(threads), 0, st, at); break;
-    }
-    return;
-  }
   const unsigned grid = (unsigned)(at.B * at.Hk * at.nsplit);
   switch (G) {
-    case 1: launch_pdl(batch_attn_kernel<DH, 1, 1>, dim3(grid), dim3(threads), 0, st, at); break;
-    case 2: launch_pdl(batch_attn_kernel<DH, 2, 1>, dim3(grid), dim3(threads), 0, st, at); break;
+    case 1: launch_pdl(batch_attn_kernel<DH, 1>, dim3(grid), dim3(threads), 0, st, at); break;
+    case 2: launch_pdl(batch_attn_kernel<DH, 2>, dim3(grid), dim3(threads), 0, st, at); break;
     default: {
       // 4 or 8 heads per kv head: the heads as rows of a tensor-core tile
       constexpr size_t smem = (size_t)kAttnWarps * 2 * kGqKeys * (DH * 2 + 16);
@@ -1791,7 +1542,20 @@ static void launch_attn_g(const AttnArgs& at, cudaStream_t st) {
     }
   }
 }
+static PaArgs prompt_args(const AttnArgs& at) {
+  PaArgs pa;
+  pa.q = at.q; pa.kcache = at.kcache; pa.vcache = at.vcache; pa.rowpos = at.seqlens; pa.rowseq = nullptr; pa.out = at.out;
+  pa.L = at.B; pa.H = at.H; pa.Hk = at.Hk; pa.S_max = at.S_max;
+  pa.scale_log2 = at.scale * 1.4426950408889634f;
+  return pa;
+}
 static int launch_attn(const AttnArgs& at, cudaStream_t st) {
+  if (at.shared_cache) {
+    // the rows are consecutive positions of one sequence
+    launch_prompt_attn(prompt_args(at), at.Dh, 1, st);
+    if (cudaGetLastError() != cudaSuccess) return fail(FSVD_ERR_CUDA, "attention kernel launch failed");
+    return 0;
+  }
   if (at.Dh == 128) launch_attn_g<128>(at, st);
   else launch_attn_g<64>(at, st);
   if (cudaGetLastError() != cudaSuccess) return fail(FSVD_ERR_CUDA, "attention kernel launch failed");
@@ -1820,7 +1584,7 @@ static int run_layer(const LayerPlan& lp, const GemmPlan& down_lift, const fsvd_
   int e;
   if (!have_xn) {
     launch_pdl(rmsnorm_rows_kernel, dim3(D.B), dim3(256), 0, st, reinterpret_cast<const __nv_bfloat16*>(x_in),
-               reinterpret_cast<const __nv_bfloat16*>(Lw.ln1_w), xn, D.d, D.eps);
+               reinterpret_cast<const __nv_bfloat16*>(Lw.ln1_w), xn, D.d, D.eps, 1, 0);
     fsvd_tile_count_launch();
   }
   if ((e = launch_gemm(lp.g[0], st))) return e;
@@ -1840,7 +1604,7 @@ static int run_layer(const LayerPlan& lp, const GemmPlan& down_lift, const fsvd_
     if ((e = launch_reduce(*r1, D.B, st))) return e;
   } else {
     launch_pdl(rmsnorm_rows_kernel, dim3(D.B), dim3(256), 0, st, mid, reinterpret_cast<const __nv_bfloat16*>(Lw.ln2_w), xn,
-               D.d, D.eps);
+               D.d, D.eps, 1, 0);
     fsvd_tile_count_launch();
   }
   for (int i = 6; i < 9; ++i)
@@ -2050,11 +1814,11 @@ static int tile_model_record(fsvd_tile_model* m, cudaStream_t st) {
     if ((e = run_layer(m->layers[l], m->down[l], D, m->lw[l], m->xbuf[l & 1], m->ws, m->L, st))) return e;
   __nv_bfloat16* xn = reinterpret_cast<__nv_bfloat16*>(m->ws + m->L.xn);
   launch_pdl(rmsnorm_rows_kernel, dim3(D.B), dim3(256), 0, st, (const __nv_bfloat16*)m->xbuf[D.n_layers & 1],
-             reinterpret_cast<const __nv_bfloat16*>(m->final_norm), xn, D.d, D.eps);
+             reinterpret_cast<const __nv_bfloat16*>(m->final_norm), xn, D.d, D.eps, 1, 0);
   fsvd_tile_count_launch();
   if ((e = launch_gemm(m->head, st))) return e;
   launch_pdl(argmax_rows_kernel, dim3(D.B), dim3(256), 0, st, (const float*)m->logits, D.vocab, m->tokens, m->token_log,
-             m->step_counter, m->seqlens, m->max_steps, D.B);
+             m->step_counter, m->seqlens, m->max_steps, D.B, 1);
   launch_pdl(bump_step_kernel, dim3(1), dim3(1), 0, st, m->step_counter);
   fsvd_tile_count_launch();
   fsvd_tile_count_launch();
@@ -2177,6 +1941,264 @@ int fsvd_tile_model_reset(fsvd_tile_model* m, void* stream) {
     return fail(FSVD_ERR_CUDA, "cudaMemsetAsync failed");
   return 0;
 }
+
+// ---- prompt pass (kernels in fsvd_prompt.cuh)
+// Rows of a pass at most; what a pass keeps per row is allocated for as many rows as the longest prompt so
+// far needed.
+constexpr int kPromptRows = 2048;
+enum PromptW { PW_QKV, PW_QU, PW_KU, PW_VU, PW_OV, PW_OU, PW_UG, PW_GU, PW_UU, PW_DV, PW_DU, PW_COUNT };
+enum PromptX { PX_XN, PX_PQ, PX_PK, PX_PV, PX_ATTN, PX_PO, PX_PUP, PX_PGATE, PX_HACT, PX_PD, PX_COUNT };
+
+struct fsvd_tile_prompt {
+  fsvd_dims D;                       // D.B = sequences
+  std::vector<fsvd_layer> lw;
+  std::vector<CUtensorMap> wmaps;    // [layer][PW_COUNT]
+  CUtensorMap xmaps[PX_COUNT];
+  const void *embed = nullptr, *final_norm = nullptr, *cos_tab = nullptr, *sin_tab = nullptr;
+  // the decode model's buffers: positions are read and advanced, the last position's token and logits go there
+  int *tokens = nullptr, *seqlens = nullptr, *step_counter = nullptr, *token_log = nullptr;
+  float* logits = nullptr;
+  int max_steps = 0, cap = 0;
+  long long wait_limit = 0;
+  char* fixed = nullptr;             // status words, normalised last rows
+  char* ws = nullptr;                // [cap] rows of everything below
+  int *rowpos = nullptr, *rowseq = nullptr;
+  __nv_bfloat16 *x = nullptr, *mid = nullptr, *xn = nullptr, *pbuf = nullptr, *qbuf = nullptr, *attn = nullptr, *hact = nullptr;
+  GemmPlan head;
+};
+
+static SyncState* prompt_sync(fsvd_tile_prompt* p) { return reinterpret_cast<SyncState*>(p->fixed); }
+static __nv_bfloat16* prompt_last(fsvd_tile_prompt* p) { return reinterpret_cast<__nv_bfloat16*>(p->fixed + al256(sizeof(SyncState))); }
+
+int fsvd_tile_prompt_destroy(fsvd_tile_prompt* p) {
+  if (!p) return 0;
+  cudaFree(p->fixed);
+  cudaFree(p->ws);
+  delete p;
+  return 0;
+}
+
+int fsvd_tile_prompt_create(const fsvd_dims* dims, const fsvd_layer* layers, const void* embed, const void* final_norm_w,
+                            const void* lm_head, const void* cos_tab, const void* sin_tab, const fsvd_tile_decode_state* st,
+                            long long wait_limit, fsvd_tile_prompt** out) {
+  const fsvd_dims& D = *dims;
+  if (int e = device_limits()) return e;
+  if (int e = check_tile_dims(D)) return e;
+  if (D.n_layers < 1 || D.vocab < 1) return fail(FSVD_ERR_ARG, "n_layers / vocab");
+  fsvd_tile_prompt* p = new fsvd_tile_prompt();
+  p->D = D;
+  p->lw.assign(layers, layers + D.n_layers);
+  p->embed = embed;
+  p->final_norm = final_norm_w;
+  p->cos_tab = cos_tab;
+  p->sin_tab = sin_tab;
+  p->tokens = st->tokens; p->seqlens = st->seqlens; p->step_counter = st->step_counter; p->token_log = st->token_log;
+  p->logits = st->logits;
+  p->max_steps = st->max_steps;
+  p->wait_limit = wait_limit;
+  const size_t fixed = al256(sizeof(SyncState)) + al256((size_t)D.B * D.d * 2);
+  cudaError_t ce = cudaMalloc(&p->fixed, fixed);
+  if (ce == cudaSuccess) ce = cudaMemset(p->fixed, 0, fixed);
+  if (ce == cudaSuccess)
+    ce = cudaFuncSetAttribute(tile_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, g_smem_optin - 1024);
+  if (ce == cudaSuccess)
+    ce = cudaFuncSetAttribute(prompt_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, g_smem_optin - 2048);
+  int e = ce == cudaSuccess ? 0 : fail(FSVD_ERR_CUDA, "allocating prompt scratch failed");
+  const int HD = D.H * D.Dh, KD = D.Hk * D.Dh;
+  p->wmaps.resize((size_t)D.n_layers * PW_COUNT);
+  for (int l = 0; l < D.n_layers && !e; ++l) {
+    const fsvd_layer& w = layers[l];
+    CUtensorMap* m = &p->wmaps[(size_t)l * PW_COUNT];
+    const struct { const void* base; int rows, K; } f[PW_COUNT] = {
+        {w.qkv_v, D.Rq + D.Rk + D.Rv, D.d}, {w.q_u, HD, D.Rq}, {w.k_u, KD, D.Rk}, {w.v_u, KD, D.Rv}, {w.o_v, D.Ro, HD}, {w.o_u, D.d, D.Ro},
+        {w.upgate_v, D.Ru + D.Rg, D.d}, {w.gate_u, D.I, D.Rg}, {w.up_u, D.I, D.Ru}, {w.down_v, D.Rd, D.I}, {w.down_u, D.d, D.Rd}};
+    for (int i = 0; i < PW_COUNT && !e; ++i) e = encode_sw128(&m[i], f[i].base, f[i].rows, f[i].K, f[i].K, kPgBoxRows);
+  }
+  if (!e) {
+    Scratch sc = {&prompt_sync(p)->status, wait_limit};
+    e = plan_gemm(p->head, lm_head, nullptr, D.vocab, D.d, D.d, prompt_last(p), nullptr, D.d, D.B, TE_STORE_F32, sc);
+    p->head.a.out = p->logits;
+  }
+  if (e) {
+    fsvd_tile_prompt_destroy(p);
+    return e;
+  }
+  *out = p;
+  return 0;
+}
+
+// Scratch for `rows` rows of a pass.
+static int prompt_reserve(fsvd_tile_prompt* p, int rows) {
+  if (rows <= p->cap) return 0;
+  int cap = 256;
+  while (cap < rows) cap *= 2;
+  const fsvd_dims& D = p->D;
+  const int HD = D.H * D.Dh, Rqkv = D.Rq + D.Rk + D.Rv, Rmlp = D.Ru + D.Rg;
+  const int pw = imax(imax(Rqkv, Rmlp), imax(D.Ro, D.Rd));
+  const size_t n = (size_t)cap;
+  const size_t bytes[] = {n * 4, n * 4, n * D.d * 2, n * D.d * 2, n * D.d * 2, n * pw * 2, n * HD * 2, n * HD * 2, n * D.I * 2};
+  size_t total = 0, off[9];
+  for (int i = 0; i < 9; ++i) {
+    off[i] = total;
+    total += al256(bytes[i]);
+  }
+  char* ws = nullptr;
+  if (cudaMalloc(&ws, total) != cudaSuccess) return fail(FSVD_ERR_CUDA, "allocating prompt scratch failed");
+  // rows past a pass's last one are multiplied too (and never stored): they have to be numbers the first time
+  if (cudaMemset(ws, 0, total) != cudaSuccess) {
+    cudaFree(ws);
+    return fail(FSVD_ERR_CUDA, "clearing prompt scratch failed");
+  }
+  cudaFree(p->ws);   // (waits for the passes that still use it)
+  p->ws = ws;
+  p->cap = cap;
+  p->rowpos = reinterpret_cast<int*>(ws + off[0]);
+  p->rowseq = reinterpret_cast<int*>(ws + off[1]);
+  __nv_bfloat16** t[] = {&p->x, &p->mid, &p->xn, &p->pbuf, &p->qbuf, &p->attn, &p->hact};
+  for (int i = 0; i < 7; ++i) *t[i] = reinterpret_cast<__nv_bfloat16*>(ws + off[2 + i]);
+  const struct { const __nv_bfloat16* base; int K, ld; } f[PX_COUNT] = {
+      {p->xn, D.d, D.d}, {p->pbuf, D.Rq, Rqkv}, {p->pbuf + D.Rq, D.Rk, Rqkv}, {p->pbuf + D.Rq + D.Rk, D.Rv, Rqkv}, {p->attn, HD, HD},
+      {p->pbuf, D.Ro, D.Ro}, {p->pbuf, D.Ru, Rmlp}, {p->pbuf + D.Ru, D.Rg, Rmlp}, {p->hact, D.I, D.I}, {p->pbuf, D.Rd, D.Rd}};
+  for (int i = 0; i < PX_COUNT; ++i)
+    if (int e = encode_sw128(&p->xmaps[i], f[i].base, cap, f[i].K, f[i].ld, kTileM)) {
+      p->cap = 0;
+      return e;
+    }
+  return 0;
+}
+
+struct PgSpec {   // one problem of a launch
+  int w, w2, x, x2, P, K, epi;
+  void* out;
+  const void* resid;
+  void* cache;
+};
+// N of a tile: the value with the shortest estimate of waves x k-blocks x (fetch of a k-block at 64
+// bytes per clock and SM, or its multiply-adds at 4096 per clock, whichever is longer).
+static int pg_tile_n(const PgSpec* sp, int n, int tiles_m, int quantum, bool two) {
+  long long best = -1;
+  int nt = quantum;
+  for (int c = kPgBoxRows; c <= (two ? kPgBufCols / 2 : kPgBufCols); c += kPgBoxRows) {
+    if (c % quantum) continue;
+    long long tiles = 0;
+    int nkb = 0;
+    for (int i = 0; i < n; ++i) {
+      tiles += (long long)tiles_m * ((sp[i].P + c - 1) / c);
+      nkb = imax(nkb, (sp[i].K + kTileK - 1) / kTileK);
+    }
+    const long long kb = imax((kTileM + c) * 128 / 64, 2 * c) * (two ? 2 : 1);
+    const long long cost = (tiles + g_sms - 1) / g_sms * (nkb * kb + 600);
+    if (best < 0 || cost < best) {
+      best = cost;
+      nt = c;
+    }
+  }
+  return nt;
+}
+static int launch_prompt_gemm(fsvd_tile_prompt* p, int layer, const PgSpec* sp, int n, int rows, cudaStream_t st) {
+  PgArgs a;
+  memset(&a, 0, sizeof(a));
+  const fsvd_dims& D = p->D;
+  a.nprob = n;
+  a.rows = rows;
+  a.tiles_m = (rows + kTileM - 1) / kTileM;
+  a.rowpos = p->rowpos; a.rowseq = p->rowseq; a.cos_tab = p->cos_tab; a.sin_tab = p->sin_tab;
+  a.Dh = D.Dh; a.HkDh = D.Hk * D.Dh; a.S_max = D.S_max;
+  a.status = &prompt_sync(p)->status;
+  a.wait_limit = p->wait_limit;
+  const bool two = sp[0].w2 >= 0;
+  const bool rope = sp[0].epi == TE_ROPE_Q;
+  const int nt = pg_tile_n(sp, n, a.tiles_m, rope ? D.Dh : kPgBoxRows, two);
+  const CUtensorMap* wm = &p->wmaps[(size_t)layer * PW_COUNT];
+  for (int i = 0; i < n; ++i) {
+    PgProblem& q = a.pr[i];
+    q.W = wm[sp[i].w];
+    q.X = p->xmaps[sp[i].x];
+    if (two) {
+      q.W2 = wm[sp[i].w2];
+      q.X2 = p->xmaps[sp[i].x2];
+    }
+    q.P = sp[i].P;
+    q.nkb = (sp[i].K + kTileK - 1) / kTileK;
+    q.nt = nt;
+    q.tile0 = a.total;
+    q.epi = sp[i].epi;
+    q.two = two ? 1 : 0;
+    q.out = sp[i].out; q.resid = sp[i].resid; q.cache = sp[i].cache;
+    a.total += a.tiles_m * ((q.P + nt - 1) / nt);
+  }
+  a.stage_bytes = (kTileM + nt) * 128 * (two ? 2 : 1);
+  a.nstages = (g_smem_optin - 4096) / a.stage_bytes;
+  if (a.nstages > kPgMaxStages) a.nstages = kPgMaxStages;
+  const int grid = a.total < g_sms ? a.total : g_sms;
+  if (launch_pdl(prompt_gemm_kernel, dim3((unsigned)grid), dim3(kPgThreads), (size_t)1024 + (size_t)a.nstages * a.stage_bytes, st, a) != cudaSuccess)
+    return fail(FSVD_ERR_CUDA, "prompt kernel launch failed");
+  fsvd_tile_count_launch();
+  return 0;
+}
+
+// prompt: device int32 [D.B, >= L] with row stride ld.
+int fsvd_tile_prompt_run(fsvd_tile_prompt* p, const int* prompt, int ld, int L, void* stream) {
+  const fsvd_dims& D = p->D;
+  cudaStream_t st = (cudaStream_t)stream;
+  const int most = kPromptRows / D.B > 1 ? kPromptRows / D.B : 1;   // positions of a pass
+  const int passes = (L + most - 1) / most, len = (L + passes - 1) / passes;
+  if (int e = prompt_reserve(p, len * D.B)) return e;
+  const int HD = D.H * D.Dh, KD = D.Hk * D.Dh, Rqkv = D.Rq + D.Rk + D.Rv;
+  auto norm = [&](const __nv_bfloat16* x, const void* w, __nv_bfloat16* out, int rows, int mul, int off) {
+    launch_pdl(rmsnorm_rows_kernel, dim3((unsigned)rows), dim3(256), 0, st, x, reinterpret_cast<const __nv_bfloat16*>(w), out, D.d, D.eps,
+               mul, off);
+    fsvd_tile_count_launch();
+  };
+  for (int off = 0; off < L; off += len) {
+    const int n = L - off < len ? L - off : len, rows = n * D.B;
+    launch_pdl(prompt_begin_kernel, dim3((unsigned)rows), dim3(128), 0, st, reinterpret_cast<const __nv_bfloat16*>(p->embed), prompt, ld,
+               off, n, (const int*)p->seqlens, p->rowpos, p->rowseq, p->x, D.d, D.vocab);
+    fsvd_tile_count_launch();
+    PaArgs pa;
+    pa.q = p->qbuf; pa.rowpos = p->rowpos; pa.rowseq = p->rowseq; pa.out = p->attn;
+    pa.L = n; pa.H = D.H; pa.Hk = D.Hk; pa.S_max = D.S_max;
+    pa.scale_log2 = 1.4426950408889634f / sqrtf((float)D.Dh);
+    for (int l = 0; l < D.n_layers; ++l) {
+      const fsvd_layer& w = p->lw[l];
+      int e = 0;
+      auto gemm = [&](std::initializer_list<PgSpec> sp) {
+        if (!e) e = launch_prompt_gemm(p, l, sp.begin(), (int)sp.size(), rows, st);
+      };
+      norm(p->x, w.ln1_w, p->xn, rows, 1, 0);
+      gemm({{PW_QKV, -1, PX_XN, -1, Rqkv, D.d, TE_STORE, p->pbuf, nullptr, nullptr}});
+      gemm({{PW_QU, -1, PX_PQ, -1, HD, D.Rq, TE_ROPE_Q, p->qbuf, nullptr, nullptr},
+            {PW_KU, -1, PX_PK, -1, KD, D.Rk, TE_ROPE_K, nullptr, nullptr, w.k_cache},
+            {PW_VU, -1, PX_PV, -1, KD, D.Rv, TE_VCACHE, nullptr, nullptr, w.v_cache}});
+      pa.kcache = reinterpret_cast<const __nv_bfloat16*>(w.k_cache);
+      pa.vcache = reinterpret_cast<const __nv_bfloat16*>(w.v_cache);
+      if (!e) launch_prompt_attn(pa, D.Dh, D.B, st);
+      gemm({{PW_OV, -1, PX_ATTN, -1, D.Ro, HD, TE_STORE, p->pbuf, nullptr, nullptr}});
+      gemm({{PW_OU, -1, PX_PO, -1, D.d, D.Ro, TE_RESID, p->mid, p->x, nullptr}});
+      norm(p->mid, w.ln2_w, p->xn, rows, 1, 0);
+      gemm({{PW_UG, -1, PX_XN, -1, D.Ru + D.Rg, D.d, TE_STORE, p->pbuf, nullptr, nullptr}});
+      gemm({{PW_GU, PW_UU, PX_PGATE, PX_PUP, D.I, D.Rg, TE_SWIGLU, p->hact, nullptr, nullptr}});
+      gemm({{PW_DV, -1, PX_HACT, -1, D.Rd, D.I, TE_STORE, p->pbuf, nullptr, nullptr}});
+      gemm({{PW_DU, -1, PX_PD, -1, D.d, D.Rd, TE_RESID, p->x, p->mid, nullptr}});
+      if (e) return e;
+    }
+    if (off + n < L) {
+      launch_pdl(advance_kernel, dim3(1), dim3(128), 0, st, p->seqlens, D.B, n);
+      fsvd_tile_count_launch();
+      continue;
+    }
+    // the last position of every sequence: final norm, head, argmax
+    norm(p->x, p->final_norm, prompt_last(p), D.B, n, n - 1);
+    if (int e = launch_gemm(p->head, st)) return e;
+    launch_pdl(argmax_rows_kernel, dim3(D.B), dim3(256), 0, st, (const float*)p->logits, D.vocab, p->tokens, p->token_log,
+               p->step_counter, p->seqlens, p->max_steps, D.B, n);
+    launch_pdl(bump_step_kernel, dim3(1), dim3(1), 0, st, p->step_counter);
+    fsvd_tile_count_launches(2);
+  }
+  if (cudaGetLastError() != cudaSuccess) return fail(FSVD_ERR_CUDA, "kernel launch failed");
+  return 0;
+}
+void* fsvd_tile_prompt_ws(fsvd_tile_prompt* p) { return p->fixed; }
 
 // Debugging aid: while a device buffer is set, every GEMM CTA planned afterwards records nine
 // %globaltimer marks (entry, set-up done, dependency met, accumulators done, cluster barrier 1,

@@ -6,6 +6,7 @@
 struct fsvd_dims;
 struct fsvd_layer;
 struct fsvd_tile_model;
+struct fsvd_tile_prompt;
 struct fsvd_exchange;
 
 // provided by fsvd_api.cu: the library's last-error text and launch counter
@@ -33,3 +34,17 @@ void fsvd_tile_model_buffers(fsvd_tile_model* m, int** tokens, int** seqlens, in
 void* fsvd_tile_model_ws(fsvd_tile_model* m);
 int fsvd_tile_model_launches_per_step(fsvd_tile_model* m);
 int fsvd_tile_model_reset(fsvd_tile_model* m, void* stream);
+
+// Prompt pass over the weights and caches of a decode model: reads and advances its positions, leaves the
+// last position's token and logits in its buffers.
+struct fsvd_tile_decode_state {
+  int *tokens, *seqlens, *step_counter, *token_log;
+  float* logits;
+  int max_steps;
+};
+int fsvd_tile_prompt_create(const fsvd_dims* dims, const fsvd_layer* layers, const void* embed, const void* final_norm_w,
+                            const void* lm_head, const void* cos_tab, const void* sin_tab, const fsvd_tile_decode_state* st,
+                            long long wait_limit, fsvd_tile_prompt** out);
+int fsvd_tile_prompt_destroy(fsvd_tile_prompt* p);
+int fsvd_tile_prompt_run(fsvd_tile_prompt* p, const int* prompt, int ld, int L, void* stream);
+void* fsvd_tile_prompt_ws(fsvd_tile_prompt* p);

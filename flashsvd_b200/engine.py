@@ -99,10 +99,9 @@ class DecodeEngine:
         cmax = 4 if dtype == torch.float32 else 8
         self.prefill_chunk = (cmax if prefill_chunk is None else max(1, min(int(prefill_chunk), cmax))) \
             if self.B == 1 else 1
-        # long prompts of a single bf16 sequence first go 128 positions per pass through the tiled
-        # tensor-core path (the same factors as 128-column GEMMs, RoPE and the cache write in their
-        # epilogues, causal attention over the rows already written)
-        self.prefill_tile = 128 if (self.B == 1 and dtype == torch.bfloat16 and not q4 and self.prefill_chunk > 1
+        # prompts of bf16 models go through the tensor-core prompt program, all positions of all
+        # sequences as the rows (128 to a tile) of dense GEMMs, unless the caller asked for chunks of 1
+        self.prefill_tile = 128 if (dtype == torch.bfloat16 and not q4 and prefill_chunk != 1
                                     and self.dims.Rg == self.dims.Ru) else 0
         self._layer_array, self._model_args = arr, (embed, final_norm, lm_head)
         self._chunk_handle = None
@@ -186,33 +185,50 @@ class DecodeEngine:
                 self._chunk_handle, self._chunk_tokens, self._chunk_seqlens, self._chunk_dims = hit
         return hit[:3]
 
+    def _prompt_program(self):
+        """Handle of the tensor-core prompt program over this engine's weights, caches and buffers."""
+        hit = self._chunks.get(self.prefill_tile)
+        if hit is None:
+            embed, final_norm, lm_head = self._model_args
+            handle = C.c_void_p()
+            with torch.cuda.device(self.device):
+                check(self.lib.fsvd_prompt_create(
+                    C.byref(self.dims), self._layer_array, embed.data_ptr(), final_norm.data_ptr(),
+                    lm_head.data_ptr(), self.cos.data_ptr(), self.sin.data_ptr(), self.handle, C.byref(handle)))
+            hit = self._chunks[self.prefill_tile] = (handle,)
+        return hit[0]
+
     def prefill(self, prompt: torch.Tensor) -> None:
-        """Feed prompt[B, L] through the decode kernels: fills the caches and leaves the first
-        generated token in ``tokens`` and its logits in ``logits``.  A single sequence goes 128
-        positions per pass (bf16; tiled tensor-core path), then 64, 32, 16 (same path) and
-        `prefill_chunk` positions per launch, causal inside a pass, each size as long as more than
-        one pass of it is left, and the rest token by token; several sequences go token by token."""
+        """Feed prompt[B, L] to the sequences: fills the caches and leaves the first generated token in
+        ``tokens`` and its logits in ``logits``.  bf16 models take all positions of all sequences
+        through the prompt program (up to 2048 rows per pass, causal per sequence).  A single fp32 or
+        int4 sequence goes `prefill_chunk` positions per launch as long as more than one chunk is
+        left and the rest token by token; several such sequences go token by token."""
         prompt = prompt.to(device=self.device, dtype=torch.int32).contiguous()
         if prompt.shape[0] != self.B:
             raise ValueError(f"prompt batch {prompt.shape[0]} != engine batch {self.B}")
         L, t0 = prompt.shape[1], 0
-        tiles = (128, 64, 32, 16) if self.prefill_tile else ()
-        sizes = [c for c in (*tiles, self.prefill_chunk) if c > 1 and L > c]
-        if self.B == 1 and sizes:
-            pos0 = int(self.seqlens[0].item())
+        Cn = self.prefill_chunk
+        stream = torch.cuda.current_stream().cuda_stream
+        if self.B == 1 and L > Cn > 1:
+            if self._pos_bound is None:
+                self._pos_bound = int(self._view("seqlens", (1,), torch.int32).item())
+            pos0 = self._pos_bound
             if pos0 + L > self.S_max:
                 raise ValueError(f"prompt of {L} tokens at position {pos0} exceeds the cache ({self.S_max})")
-            stream = torch.cuda.current_stream().cuda_stream
-            for Cn in sizes:
-                if L - t0 <= Cn:
-                    continue
-                handle, tokens, seqlens = self._chunk_model(Cn)
-                offs = torch.arange(Cn, device=self.device, dtype=torch.int32)
-                while L - t0 > Cn:
-                    tokens.copy_(prompt[0, t0:t0 + Cn])
-                    seqlens.copy_(offs + (pos0 + t0))
-                    check(self.lib.fsvd_model_step(handle, 1, stream))
-                    t0 += Cn
+        if self.prefill_tile and L > 1:
+            handle = self._prompt_program()
+            self._reserve_positions(L)
+            check(self.lib.fsvd_prompt_run(handle, prompt.data_ptr(), L, L, stream))
+            return
+        if self.B == 1 and L > Cn > 1:
+            handle, tokens, seqlens = self._chunk_model(Cn)
+            offs = torch.arange(Cn, device=self.device, dtype=torch.int32)
+            while L - t0 > Cn:
+                tokens.copy_(prompt[0, t0:t0 + Cn])
+                seqlens.copy_(offs + (pos0 + t0))
+                check(self.lib.fsvd_model_step(handle, 1, stream))
+                t0 += Cn
             self.seqlens.fill_(pos0 + t0)
             self._pos_bound = pos0 + t0
         tok = self.tokens
@@ -237,7 +253,7 @@ class DecodeEngine:
         return int(st.value)
 
     def close(self) -> None:
-        for hit in getattr(self, "_chunks", {}).values():
+        for hit in getattr(self, "_chunks", {}).values():   # before the model they read and write
             if hit[0].value:
                 self.lib.fsvd_model_destroy(hit[0])
         self._chunks = {}

@@ -242,6 +242,18 @@ int fsvd_model_destroy(fsvd_model* m);
 /* Enqueue n_steps greedy decode steps: one kernel launch per step for B <= 8, one CUDA graph launch
  * per step (captured by fsvd_model_create) for B > 8. */
 int fsvd_model_step(fsvd_model* m, int n_steps, void* stream);
+/* Prompt program of a decode model (bf16 factors, equal gate / up ranks; dims, weights and caches are
+ * the decode model's): fsvd_prompt_run feeds tokens[B, length] (device int32, rows row_stride apart) to
+ * the B sequences at positions seqlens[b] .. seqlens[b] + length - 1, up to 2048 rows per pass, fills the
+ * caches, and leaves the token sampled after the last position in the decode model's tokens / token_log,
+ * its logits in logits, and seqlens / step_counter advanced by length / 1.  The scratch grows with the
+ * longest prompt (allocated by the first run that needs it).  fsvd_model_status, fsvd_model_reset_sync
+ * and fsvd_model_destroy take a prompt program too; it is destroyed before the decode model.  The
+ * reference fills the cache with its prefill kernels (kernels/flashsvdropeattn.py:67-427). */
+int fsvd_prompt_create(const fsvd_dims* dims, const fsvd_layer* layers, const void* embed,
+                       const void* final_norm_w, const void* lm_head, const void* cos_tab,
+                       const void* sin_tab, fsvd_model* decode, fsvd_model** out);
+int fsvd_prompt_run(fsvd_model* prompt, const int* tokens, int row_stride, int length, void* stream);
 /* Device buffers: tokens[B] (in: token to feed, out: sampled token), seqlens[B],
  * token_log[max_steps,B], step_counter[1], logits[B,vocab] fp32; `hidden` is the library's internal
  * hidden-state buffer between layers ([B,d] in the model dtype), exposed for debugging. */
