@@ -91,8 +91,11 @@ __device__ __forceinline__ uint32_t umma_idesc(int N) {
 
 // Cluster barrier (all threads of all CTAs of the cluster) and a store into the shared memory of
 // the cluster's CTA `rank` at the same offset as the local address `addr`.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  cluster_arrive();
+  cluster_wait();
 }
 __device__ __forceinline__ void st_cluster_v4(uint32_t addr, uint32_t rank, float x, float y, float z, float w) {
   uint32_t remote;

@@ -57,7 +57,7 @@
 
 namespace fsvd_tile {
 
-constexpr int kThreads = 128;        // 4 warps: warp w reads accumulator lanes 32 w .. 32 w + 31
+constexpr int kThreads = 256;        // 8 warps: warp w reads accumulator lanes 32 (w % 4) .. + 31, every other 16 columns
 constexpr int kWTileBytes = kTileM * kTileK * 2;   // 16 KB
 constexpr int kMaxStages = 8;
 constexpr int kMaxSegs = 8;           // K segments of a tile = CTAs of a cluster (portable size)
@@ -74,12 +74,14 @@ enum TileEpi : int {
 };
 
 struct GemmArgs {
-  int P, K, B, N;          // factor rows, reduction length, batch rows, batch rounded up to 16
+  int P, K, B, N;          // factor rows, reduction length, batch rows, batch columns of a tile (a multiple of 16)
   int tiles, segs, kbs;    // row tiles, K segments, k-blocks per segment
+  int nh;                  // CTAs that share a row tile's batch columns (N each): 1 or 2
   int nkb;                 // k-blocks in all
   int nstages, two, epi;
   uint32_t tmem_cols;      // power of two >= 32
   int cpo;                 // batch columns finished by each CTA of a tile's cluster: ceil(N / segs) rounded up to 4
+  uint32_t recv_off;       // byte offset of the partial sums this CTA receives; 0: they take the ring's place
   void* out;
   const void* resid;
   void* cache;             // TE_ROPE_K / TE_VCACHE: [rows, S_max, Hk, Dh]
@@ -111,10 +113,15 @@ struct GemmGroup {
 };
 
 // ------------------------------------------------------------------------------- GEMM kernel
-// grid = (tiles, segs, problems).  Dynamic shared memory: [1 KB slack for alignment][NS stages].
-__global__ void __launch_bounds__(kThreads) tile_gemm_kernel(const __grid_constant__ GemmGroup grp) {
+// grid = (tiles x nh, segs, problems).  Dynamic shared memory: [1 KB slack for alignment][NS stages][partial sums].
+// What bounds it: the factor stream, then, launch by launch, the chain dependency -> activations ->
+// multiply -> exchange -> epilogue.  Per launch after its dependency (7B shape, us, median of the CTAs
+// past the epilogue): 128 columns 22 -> 12 (lifts with rotary 27 -> 12, gate / up 36 -> 12), 16 columns
+// 4.4 -> 4.2; the step of 4 layers: 128 sequences 8.13 -> 6.50 ms, 32 sequences 5.32 -> 4.97 ms, 8 sequences of
+// the 70B shape 2.95 -> 2.88 ms.
+__global__ void __launch_bounds__(kThreads, 3) tile_gemm_kernel(const __grid_constant__ GemmGroup grp) {
   const GemmArgs& a = grp.args[blockIdx.z];
-  if ((int)blockIdx.x >= a.tiles || (int)blockIdx.y >= a.segs) return;
+  if ((int)blockIdx.x >= a.tiles * a.nh || (int)blockIdx.y >= a.segs) return;
   const CUtensorMap& mapA = grp.maps[blockIdx.z][0];
   const CUtensorMap& mapA2 = grp.maps[blockIdx.z][1];
   const CUtensorMap& mapX = grp.maps[blockIdx.z][2];
@@ -125,7 +132,8 @@ __global__ void __launch_bounds__(kThreads) tile_gemm_kernel(const __grid_consta
   __shared__ int giveup_sh;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int tile = blockIdx.x, seg = blockIdx.y;
+  const int tile = a.nh == 2 ? blockIdx.x >> 1 : blockIdx.x, seg = blockIdx.y;
+  const int bcol = a.nh == 2 ? (int)(blockIdx.x & 1) * a.N : 0;   // first batch column
   tmark(a, 0);
   const int N = a.N, NS = a.nstages;
   const uint32_t xbytes = (uint32_t)N * 128u;
@@ -155,11 +163,12 @@ __global__ void __launch_bounds__(kThreads) tile_gemm_kernel(const __grid_consta
   const uint32_t tmem = tmem_slot;
   tmark(a, 1);
   pdl_launch_dependents();
+  if (a.recv_off) cluster_arrive();   // "this CTA runs": its receive buffer may be written from now on
 
   const int kb0 = seg * a.kbs, kb1 = min(a.nkb, kb0 + a.kbs);
   const int nit = kb1 - kb0;
 
-  if (warp != 1) {
+  if (warp != 1 && warp < 4) {
     if (lane == 0) {
       // ---- producers: TMA copies of the stage operands.  One thread sustains about 24 GB/s of
       // copies (wait, arm, issue per box), so three threads (warps 0, 2, 3) share the stages.  A
@@ -194,8 +203,8 @@ __global__ void __launch_bounds__(kThreads) tile_gemm_kernel(const __grid_consta
           if (a.two) tma_box_2d(dst + kWTileBytes, &mapA2, kcol, tile * kTileM, fb);
         }
         dst += (uint32_t)kWTileBytes * (a.two ? 2u : 1u);
-        tma_box_2d(dst, &mapX, kcol, 0, fb);
-        if (a.two) tma_box_2d(dst + xbytes, &mapX2, kcol, 0, fb);
+        tma_box_2d(dst, &mapX, kcol, bcol, fb);
+        if (a.two) tma_box_2d(dst + xbytes, &mapX2, kcol, bcol, fb);
       }
     }
     __syncwarp();
@@ -235,50 +244,84 @@ __global__ void __launch_bounds__(kThreads) tile_gemm_kernel(const __grid_consta
   pdl_wait();
   tmark(a, 2);
   const unsigned push_seq = a.epi == TE_PUSH ? *reinterpret_cast<const volatile unsigned*>(a.ex_seq) : 0u;
-  // the residual rows this CTA will add have usually left L2 since they were written (a layer's
-  // factors stream through in between): ask for them now, the epilogue is several microseconds away
-  if (a.epi == TE_RESID && lane == 0) {
-    const int prow = tile * kTileM + warp * 32;
-    if (prow < a.P)
-      for (int sl = 0; sl < a.cpo; ++sl) {
-        const int b = seg * a.cpo + sl;
-        if (b < a.B)
-          asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const __nv_bfloat16*>(a.resid) + (size_t)b * a.P + prow));
+
+  // ---- this thread's share of the epilogue: row r of the tile, four batch columns at a time, every
+  // ng-th group of four of the CTA's slice.  RoPE finishes rows j and j + Dh/2 of a head together, so
+  // half as many rows are shared out over twice as many column groups.
+  const int cpo = a.cpo;                     // batch columns finished by each CTA of the cluster
+  const int half = a.Dh >> 1;
+  const bool rope = a.epi == TE_ROPE_Q || a.epi == TE_ROPE_K;
+  const int er = rope ? tid & (kTileM / 2 - 1) : tid & (kTileM - 1);
+  const int j = rope ? er & (half - 1) : 0;  // (Dh is 64 or 128)
+  const int r = rope ? 2 * (er - j) + j : er;
+  const int p = tile * kTileM + r;           // factor row
+  const int sl0 = 4 * (rope ? tid >> 6 : tid >> 7), sl_step = rope ? 16 : 8;
+  const bool work = p < a.P;
+  // Operands of four columns that do not depend on the accumulators: residual elements, or the
+  // position and the rotary pair.  Those of the first four are requested before the accumulators are
+  // complete, those of the next four before the arithmetic of the four at hand.
+  auto operands = [&](int sl, uint32_t (&x)[4], int (&pos)[4]) {
+    const int b0 = bcol + seg * cpo + sl;
+    if (!work || sl >= cpo || b0 >= a.B) return;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int b = min(b0 + i, a.B - 1);
+      if (a.epi == TE_RESID) {
+        x[i] = reinterpret_cast<const unsigned short*>(a.resid)[(size_t)b * a.P + p];
+      } else {
+        pos[i] = a.seqlens[b];
+        if (rope) {
+          const size_t t = (size_t)min(pos[i], a.S_max - 1) * half + j;
+          x[i] = reinterpret_cast<const unsigned short*>(a.cos_tab)[t] |
+                 (uint32_t) reinterpret_cast<const unsigned short*>(a.sin_tab)[t] << 16;
+        }
       }
-  }
+    }
+  };
+  const int epi = a.epi, segs = a.segs, B = a.B, P = a.P;   // (indexed constant loads: once, not per column)
+  const bool two = a.two != 0;
+  void* const out = a.out;
+  const bool has_operands = rope || a.epi == TE_RESID || a.epi == TE_VCACHE;
+  uint32_t xn[4] = {0u, 0u, 0u, 0u};
+  int posn[4] = {0, 0, 0, 0};
+  if (has_operands) operands(sl0, xn, posn);
+
   bool have = nit > 0 ? wait_bar(accum, 0u, giveup, a.status, a.wait_limit, DS_BARRIER_TIMEOUT) : false;
   have = __all_sync(0xffffffffu, have);
   tc_fence_after();
   tmark(a, 3);
 
-  const int r = tid;                       // accumulator lane = row of the tile
-  const int p = tile * kTileM + r;         // factor row
-  const uint32_t trow = tmem + ((uint32_t)(warp * 32) << 16);
-  const int nacc = a.two ? 2 : 1;
-  const int cpo = a.cpo;                   // batch columns finished by each CTA of the cluster
-
   // ---- the K segments of a tile are the CTAs of one cluster (rank = segment).  CTA j finishes the
   // batch columns [j cpo, (j + 1) cpo) (cpo a multiple of 4): every CTA sends its partial sums of
-  // those columns to CTA j's shared memory, [accumulator][segment][row][cpo] floats, four columns per
-  // 16-byte store; the ring is free for that once every CTA of the cluster has its accumulators
-  // (first cluster barrier), and the sums are complete after the second.  Every CTA reaches both
-  // barriers, whatever happened before.
-  float* recv = reinterpret_cast<float*>(base_ptr);
-  const uint32_t recv_u32 = base;
-  cluster_sync();
+  // those columns to CTA j's shared memory, [accumulator][segment][group of four columns][row] x 16
+  // bytes: the lanes of a warp hold consecutive rows, so a store (and the load below) covers 512
+  // consecutive bytes.  (With the columns of a row next to each other instead, a warp's store hit
+  // the same banks up to 32 times: 10 us of sending and 15 us of epilogue per launch at 128 columns.)
+  // Where the buffer has its own place the CTAs of the cluster only have to be running before the
+  // first store; where it reuses the ring every CTA must have its accumulators.  The sums are
+  // complete after the second barrier.  Every CTA reaches both, whatever happened before.
+  const float4* recv = reinterpret_cast<const float4*>(base_ptr + a.recv_off);
+  const uint32_t recv_u32 = base + a.recv_off;
+  const int nacc = a.two ? 2 : 1, cq = cpo >> 2;
+  if (!a.recv_off) cluster_arrive();
+  cluster_wait();
   tmark(a, 4);
   if (have) {
+    const int arow = (warp & 3) * 32 + lane;   // accumulator lane = row of the tile
+    const uint32_t trow = tmem + ((uint32_t)((warp & 3) * 32) << 16);
     for (int acc = 0; acc < nacc; ++acc) {
-      for (int c0 = 0; c0 < N; c0 += 16) {
+      for (int c0 = (warp >> 2) * 16; c0 < N; c0 += 32) {
         float v[16];
         tc_ld16(trow + (uint32_t)(acc * N + c0), v);
+        int owner = c0 / cpo, q = (c0 - owner * cpo) >> 2;
 #pragma unroll
         for (int q4 = 0; q4 < 4; ++q4) {
-          const int col = c0 + 4 * q4;
-          const int owner = col / cpo, slot = col - owner * cpo;
-          if (owner < a.segs)
-            st_cluster_v4(recv_u32 + (uint32_t)(((((acc * a.segs + seg) * kTileM + r) * cpo) + slot) * 4), (uint32_t)owner,
-                          v[4 * q4], v[4 * q4 + 1], v[4 * q4 + 2], v[4 * q4 + 3]);
+          const uint32_t dst = recv_u32 + (uint32_t)((((acc * a.segs + seg) * cq + q) * kTileM + arow) * 16);
+          if (owner < a.segs) st_cluster_v4(dst, (uint32_t)owner, v[4 * q4], v[4 * q4 + 1], v[4 * q4 + 2], v[4 * q4 + 3]);
+          if (++q == cq) {
+            q = 0;
+            ++owner;
+          }
         }
       }
     }
@@ -287,96 +330,83 @@ __global__ void __launch_bounds__(kThreads) tile_gemm_kernel(const __grid_consta
   cluster_sync();
   tmark(a, 6);
 
-  if (!*giveup && have && p < a.P) {
-    const int half = a.Dh >> 1;
-    const bool rope = a.epi == TE_ROPE_Q || a.epi == TE_ROPE_K;
-    const int j = rope ? p % a.Dh : 0;
-    const bool lower = !rope || j < half;      // RoPE: the thread of row j < Dh/2 finishes rows j and j + Dh/2
-    for (int sl = 0; sl < cpo && lower; sl += 4) {
-      const int b0 = seg * cpo + sl;
-      if (b0 >= a.B) break;
+  if (!*giveup && have && work) {
+    for (int sl = sl0; sl < cpo; sl += sl_step) {
+      const int b0 = bcol + seg * cpo + sl;
+      if (b0 >= B) break;
+      uint32_t x[4];
+      int pos[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) x[i] = xn[i], pos[i] = posn[i];
+      if (has_operands) operands(sl + sl_step, xn, posn);
       // sums over the segments, in segment order, of four columns (and of the second accumulator,
       // or of the RoPE partner row)
       float v[4] = {0.f, 0.f, 0.f, 0.f}, u[4] = {0.f, 0.f, 0.f, 0.f};
-      for (int sg = 0; sg < a.segs; ++sg) {
-        const float4 t = *reinterpret_cast<const float4*>(recv + ((size_t)(sg * kTileM + r) * cpo + sl));
+      const float4* src = recv + (sl >> 2) * kTileM + r;
+      for (int sg = 0; sg < segs; ++sg) {
+        const float4 t = src[sg * cq * kTileM];
         v[0] += t.x; v[1] += t.y; v[2] += t.z; v[3] += t.w;
       }
-      if (a.two || rope) {
-        for (int sg = 0; sg < a.segs; ++sg) {
-          const size_t row2 = a.two ? (size_t)((a.segs + sg) * kTileM + r) : (size_t)(sg * kTileM + r + half);
-          const float4 t = *reinterpret_cast<const float4*>(recv + (row2 * cpo + sl));
+      if (two || rope) {
+        src += two ? segs * cq * kTileM : half;
+        for (int sg = 0; sg < segs; ++sg) {
+          const float4 t = src[sg * cq * kTileM];
           u[0] += t.x; u[1] += t.y; u[2] += t.z; u[3] += t.w;
         }
       }
-      // One compact code path per epilogue kind (this code runs once per CTA, from a cold
-      // instruction cache: the fewer lines it spans, the sooner it is through); within a kind the
-      // operands of the four columns are loaded first, then come the arithmetic and the stores.
-      const int nb = min(4, a.B - b0);
-      const size_t o0 = (size_t)b0 * a.P + p;
-      if (a.epi == TE_STORE) {
+      // One compact code path per epilogue kind (this code often runs once per CTA, from a cold
+      // instruction cache: the fewer lines it spans, the sooner it is through).
+      const int nb = min(4, B - b0);
+      const size_t o0 = (size_t)b0 * P + p;
+      if (epi == TE_STORE) {
 #pragma unroll
         for (int i = 0; i < 4; ++i)
-          if (i < nb) stbf(a.out, o0 + (size_t)i * a.P, v[i]);
-      } else if (a.epi == TE_RESID) {
-        float res[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) res[i] = ldbf(a.resid, o0 + (size_t)min(i, nb - 1) * a.P);
+          if (i < nb) stbf(out, o0 + (size_t)i * P, v[i]);
+      } else if (epi == TE_RESID) {
 #pragma unroll
         for (int i = 0; i < 4; ++i)
-          if (i < nb) stbf(a.out, o0 + (size_t)i * a.P, res[i] + rnd(v[i]));
-      } else if (a.epi == TE_PUSH) {
+          if (i < nb) stbf(out, o0 + (size_t)i * P, __uint_as_float(x[i] << 16) + rnd(v[i]));
+      } else if (epi == TE_PUSH) {
         // the same rounded partial sums into slot [parity][this rank] of every rank's region
         // (peer stores over NVLink; the rank's own region among them)
         for (int q = 0; q < a.ex.world; ++q) {
           unsigned char* dst = fsvd_exch::slot_ptr(a.ex, q, push_seq & 1u, a.ex.rank);
 #pragma unroll
           for (int i = 0; i < 4; ++i)
-            if (i < nb) stbf(dst, o0 + (size_t)i * a.P, v[i]);
+            if (i < nb) stbf(dst, o0 + (size_t)i * P, v[i]);
         }
-      } else if (a.epi == TE_SWIGLU) {
+      } else if (epi == TE_SWIGLU) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const float g = rnd(v[i]), up = rnd(u[i]);
           const float sg = rnd(g / (1.0f + expf(-g)));
-          if (i < nb) stbf(a.out, o0 + (size_t)i * a.P, sg * up);
+          if (i < nb) stbf(out, o0 + (size_t)i * P, sg * up);
         }
-      } else if (a.epi == TE_STORE_F32) {
+      } else if (epi == TE_STORE_F32) {
 #pragma unroll
         for (int i = 0; i < 4; ++i)
-          if (i < nb) reinterpret_cast<float*>(a.out)[o0 + (size_t)i * a.P] = rnd(v[i]);
+          if (i < nb) reinterpret_cast<float*>(out)[o0 + (size_t)i * P] = rnd(v[i]);
       } else {
-        // value cache / rotary epilogues: position of every column, tables, then the stores
-        int pos[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) pos[i] = a.seqlens[min(b0 + i, a.B - 1)];
-        float cs[4], sn[4];
-        if (rope) {
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const int pt = min(pos[i], a.S_max - 1);
-            cs[i] = ldbf(a.cos_tab, (size_t)pt * half + j);
-            sn[i] = ldbf(a.sin_tab, (size_t)pt * half + j);
-          }
-        }
+        // value cache / rotary epilogues
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const int b = b0 + i;
           if (i >= nb) continue;
-          if (pos[i] >= a.S_max && a.epi != TE_ROPE_Q) {
+          if (pos[i] >= a.S_max && epi != TE_ROPE_Q) {
             atomicCAS(a.status, (int)DS_OK, (int)DS_CACHE_FULL);
             continue;
           }
           const size_t oc = ((size_t)(a.shared_cache ? 0 : b) * a.S_max + pos[i]) * (size_t)a.HkDh + p;
-          if (a.epi == TE_VCACHE) {
+          if (epi == TE_VCACHE) {
             stbf(a.cache, oc, v[i]);
           } else {
+            const float cs = __uint_as_float(x[i] << 16), sn = __uint_as_float(x[i] & 0xffff0000u);
             const float x1 = rnd(v[i]), x2 = rnd(u[i]);
-            const float o1 = rnd(rnd(x1 * cs[i]) - rnd(x2 * sn[i]));
-            const float o2 = rnd(rnd(x2 * cs[i]) + rnd(x1 * sn[i]));
-            if (a.epi == TE_ROPE_Q) {
-              stbf(a.out, o0 + (size_t)i * a.P, o1);
-              stbf(a.out, o0 + (size_t)i * a.P + half, o2);
+            const float o1 = rnd(rnd(x1 * cs) - rnd(x2 * sn));
+            const float o2 = rnd(rnd(x2 * cs) + rnd(x1 * sn));
+            if (epi == TE_ROPE_Q) {
+              stbf(out, o0 + (size_t)i * P, o1);
+              stbf(out, o0 + (size_t)i * P + half, o2);
             } else {
               stbf(a.cache, oc, o1);
               stbf(a.cache, oc + half, o2);
@@ -1219,10 +1249,14 @@ static int plan_gemm(GemmPlan& g, const void* W, const void* W2, int P, int K, i
                      int ldx, int B, int epi, const Scratch& sc, int force_segs = 0) {
   if (int e = device_limits()) return e;
   memset(&g, 0, sizeof(g));
-  const int N = round16(B);
   GemmArgs& a = g.a;
-  a.P = P; a.K = K; a.B = B; a.N = N;
   a.tiles = (P + kTileM - 1) / kTileM;
+  // Wide batches: two CTAs take half of the columns each where the row tiles alone leave SMs idle (8 K
+  // segments do not make up for it), or where two accumulators of all columns take the whole shared
+  // memory of an SM and with it the K split.  The second CTA finds the factor tile in L2.
+  a.nh = B > 64 && (epi == TE_SWIGLU || (epi == TE_STORE && a.tiles * kMaxSegs < g_sms)) ? 2 : 1;
+  const int N = round16((B + a.nh - 1) / a.nh);
+  a.P = P; a.K = K; a.B = B; a.N = N;
   a.nkb = (K + kTileK - 1) / kTileK;
   a.two = W2 ? 1 : 0;
   a.epi = epi;
@@ -1234,7 +1268,7 @@ static int plan_gemm(GemmPlan& g, const void* W, const void* W2, int P, int K, i
   size_t smem = 0;
   int cap = kMaxSegs;
   for (int attempt = 0; attempt < 2; ++attempt) {
-    split_k(a.tiles, a.nkb, g_sms, a.segs, a.kbs);
+    split_k(a.tiles * a.nh, a.nkb, g_sms, a.segs, a.kbs);
     if (force_segs > 0) {   // the caller wants this many segments (problems of one grouped launch)
       const int want = force_segs < a.nkb ? force_segs : a.nkb;
       a.kbs = (a.nkb + want - 1) / want;
@@ -1257,22 +1291,32 @@ static int plan_gemm(GemmPlan& g, const void* W, const void* W2, int P, int K, i
     if (ns < 1) return fail(FSVD_ERR_UNSUPPORTED, "shared memory too small for one stage");
     a.nstages = ns;
     smem = 1024 + (size_t)ns * stage;
-    // the ring is reused for the partial sums the cluster's CTAs send each other
+    // the partial sums the cluster's CTAs send each other: in a place of their own (then a CTA may send
+    // before its peers have finished) where that leaves two CTAs per SM and the launch, the three lifts
+    // of a layer together, resident at once; else in the ring's
     const size_t recv = (size_t)nacc * a.segs * a.cpo * kTileM * 4;
-    if (smem < 1024 + recv) smem = 1024 + recv;
+    const bool lift = epi == TE_ROPE_Q || epi == TE_ROPE_K || epi == TE_VCACHE;
+    const int per_sm = (int)((size_t)(228 * 1024) / (smem + recv + 1280));
+    if (smem + recv <= 112 * 1024 && (!lift || per_sm * g_sms >= 3 * a.tiles * a.segs)) {
+      a.recv_off = (uint32_t)(ns * stage);
+      smem += recv;
+    } else {
+      a.recv_off = 0;
+      if (smem < 1024 + recv) smem = 1024 + recv;
+    }
     // co-resident CTAs must not ask for more than the 512 tensor-memory columns of an SM
     const size_t floor_smem = (size_t)232448 / (512 / cols + 1) + 1024;
     if (smem < floor_smem) smem = floor_smem;
     // one CTA per SM and more CTAs than SMs would run in two waves: take fewer segments instead
-    if (attempt == 0 && smem > 113 * 1024 && a.tiles * a.segs > g_sms && a.segs > 1) {
-      cap = g_sms / a.tiles > 0 ? g_sms / a.tiles : 1;
+    if (attempt == 0 && smem > 113 * 1024 && a.tiles * a.nh * a.segs > g_sms && a.segs > 1) {
+      cap = g_sms / (a.tiles * a.nh) > 0 ? g_sms / (a.tiles * a.nh) : 1;
       continue;
     }
     break;
   }
   if (smem > (size_t)g_smem_optin - 1024) return fail(FSVD_ERR_UNSUPPORTED, "shared memory plan exceeds the device limit");
   g.smem = smem;
-  g.grid = dim3((unsigned)a.tiles, (unsigned)a.segs);
+  g.grid = dim3((unsigned)(a.tiles * a.nh), (unsigned)a.segs);
   a.status = sc.status;
   a.wait_limit = sc.wait_limit;
   a.trace = (g_tile_trace_epi < 0 || g_tile_trace_epi == epi) ? g_tile_trace : nullptr;

@@ -91,6 +91,17 @@ def test_decode_layer_tiles_ragged_ranks(dev):
     assert rel_linf(out, ref) <= TOL
 
 
+@pytest.mark.parametrize("B", [64, 65, 81, 127])
+def test_decode_layer_tiles_wide_batches_in_halves(dev, B):
+    """From 65 sequences on two CTAs take half of a tile's columns each (48 + 17, 48 + 33, 64 + 63 here, and
+    64 in one piece) and a CTA's column slice ends inside a group of four."""
+    shape = O.Shape(d=256, H=4, Hk=2, Dh=64, I=392, Rq=72, Rk=40, Rv=24, Ro=88, Rg=56, Ru=56, Rd=104, vocab=300, n_layers=1)
+    out, ref, pk, kc_o, vc_o = _layer_case(dev, shape, B, 19, S_max=24)
+    assert rel_linf(pk["k_cache"], kc_o) <= TOL
+    assert rel_linf(pk["v_cache"], vc_o) <= TOL
+    assert rel_linf(out, ref) <= TOL
+
+
 @pytest.mark.parametrize("B", [16, 32])
 def test_decode_layer_tiles_7b_shape(dev, B):
     # one Llama-2-7B-shaped layer, ranks 1024 / 1488, 512 cached positions
