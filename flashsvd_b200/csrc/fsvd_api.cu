@@ -236,6 +236,12 @@ static WsLayout ws_layout(const fsvd_dims& D) {
   return L;
 }
 
+// Running argmax keys of a model's rows (at most 8): behind the barrier words, in the same 256 bytes.
+static_assert(sizeof(SyncState) <= 128);
+static unsigned long long* argmax_keys(char* ws, const WsLayout& L) {
+  return reinterpret_cast<unsigned long long*>(ws + L.sync + 128);
+}
+
 // ------------------------------------------------------------------------------- builder
 struct MapPair {
   unsigned char m[2][128];
@@ -1244,12 +1250,13 @@ int fsvd_model_create(const fsvd_dims* dims, const fsvd_layer* layers, const voi
     s.eps = D.eps;
     s.epi = EPI_STORE;
     s.out = m->logits;
+    s.best = argmax_keys(m->ws, m->L);
   }
   {
     Stage s = b.blank();
     s.type = ST_ARGMAX;
     s.flags = 0;
-    s.vl_src = m->logits;
+    s.best = argmax_keys(m->ws, m->L);
     s.vocab = D.vocab;
     s.tokens = m->tokens;
     s.token_log = m->token_log;
@@ -1395,7 +1402,7 @@ int fsvd_model_reset_sync(fsvd_model* m, void* stream) {
   if (!m) return fail(FSVD_ERR_ARG, "null model");
   if (m->prompt) return fsvd_workspace_clear_status(fsvd_tile_prompt_ws(m->prompt), stream);
   if (m->tile) return fsvd_tile_model_reset(m->tile, stream);
-  CUDA_TRY(cudaMemsetAsync(m->ws + m->L.sync, 0, sizeof(SyncState), (cudaStream_t)stream));
+  CUDA_TRY(cudaMemsetAsync(m->ws + m->L.sync, 0, al256(sizeof(SyncState)), (cudaStream_t)stream));   // (and the argmax keys)
   CUDA_TRY(cudaMemsetAsync(m->ws + m->L.counters, 0, kCounterBytes, (cudaStream_t)stream));
   return 0;
 }

@@ -824,6 +824,37 @@ __device__ __forceinline__ void q4_box(uint32_t wb, uint32_t sb, uint32_t xq, in
   }
 }
 
+// Order of (value, index) pairs as one integer: larger values first, then lower indices; -0 = +0.  A
+// NaN never wins (0 = nothing yet).
+__device__ __forceinline__ unsigned long long argmax_key(float v, int index) {
+  if (!(v == v)) return 0ull;
+  const uint32_t u = __float_as_uint(v == 0.f ? 0.f : v);
+  const uint32_t m = (u >> 31) ? ~u : (u | 0x80000000u);
+  return ((unsigned long long)m << 32) | (uint32_t)~index;
+}
+// The logits of this CTA (one operand, one K segment) once more from the warps' partial sums: the best
+// of every 16 rows goes into the batch row's key.  (Not inlined: inside the epilogue loop it costs the
+// interpreter spills.)
+template <typename T>
+static __device__ __noinline__ void best_logits(const Stage& st, const float* part, int nu, int first, int KK, int tid) {
+  const int rowsB = kUnitRows * st.B, r = tid & 15;
+  const unsigned half_warp = 0xffffu << (tid & 16);
+  for (int o = tid; o < nu * rowsB; o += kConsThreads) {   // multiples of 16: half warps stay together
+    const int j = qdiv(o, rowsB), b = (o - j * rowsB) >> 4;
+    const int p = (first + j * (int)gridDim.x) * kUnitRows + r;
+    const float* src = part + (size_t)j * KK * rowsB + b * 16 + r;
+    float sum = 0.f;
+    for (int k = 0; k < KK; ++k) sum += src[(size_t)k * rowsB];
+    unsigned long long key = p < st.P ? argmax_key(TT<T>::rnd(sum), p) : 0ull;
+#pragma unroll
+    for (int s = 8; s > 0; s >>= 1) {
+      const unsigned long long other = __shfl_xor_sync(half_warp, key, s);
+      if (other > key) key = other;
+    }
+    if (r == 0 && key) atomicMax(st.best + b, key);
+  }
+}
+
 // Per-stage context handed to the stage functions.
 struct StageCtx {
   int s;
@@ -1048,6 +1079,7 @@ __device__ __forceinline__ int gemv_stage(const Stage& st, const StageCtx cx) {
       for (int k2 = 0; k2 < KK; ++k2) sum1 += src[(size_t)(KK + k2) * rowsB];
     gemv_epilogue<T>(st, p, b, seg, sum0, sum1, ax);
   }
+  if (st.best) best_logits<T>(st, cx.part, bp.nu, bp.first, KK, tid);
   trace_mark(cx.trow, 11);
   return bp.nbox;
 }
@@ -1381,58 +1413,18 @@ __device__ __forceinline__ void run_embed(const Stage& st, int gtid, int gthread
   }
 }
 
-// CTA 0 only.  Lowest index wins among equal maxima.
-static __device__ __forceinline__ void run_argmax(const Stage& st, float* redv, int* redi, int tid,
-                                           int nthreads) {
-  const int V = st.vocab, B = st.B;
-  const int warp = tid >> 5, lane = tid & 31, nwarps = nthreads >> 5;
-  const float* logits = reinterpret_cast<const float*>(st.vl_src);
-  int step = *st.step_counter;
-  for (int b = 0; b < B; ++b) {
-    float best = -INFINITY;
-    int bi = 0x7fffffff;
-    for (int v0 = tid; v0 < V; v0 += nthreads * 8) {
-      float x[8];
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const int v = v0 + q * nthreads;
-        x[q] = v < V ? __ldcg(logits + (size_t)b * V + v) : -INFINITY;
-      }
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const int v = v0 + q * nthreads;
-        if (v < V && (x[q] > best || (x[q] == best && v < bi))) {
-          best = x[q];
-          bi = v;
-        }
-      }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-      const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-      if (ob > best || (ob == best && oi < bi)) {
-        best = ob;
-        bi = oi;
-      }
-    }
-    if (lane == 0) {
-      redv[warp] = best;
-      redi[warp] = bi;
-    }
-    cons_sync();
-    if (tid == 0) {
-      for (int i = 1; i < nwarps; ++i)
-        if (redv[i] > best || (redv[i] == best && redi[i] < bi)) {
-          best = redv[i];
-          bi = redi[i];
-        }
-      if (bi == 0x7fffffff) bi = 0;
-      st.tokens[b] = bi;
-      if (st.token_log && step < st.max_steps) st.token_log[(size_t)step * B + b] = bi;
-      if (st.seqlens_rw) st.seqlens_rw[b] += 1;
-    }
-    cons_sync();
+// CTA 0 only, threads 0 .. B - 1 (one warp): the lm_head stage has left the winners in st.best.  (Scanning
+// the logits here took one CTA 10 us per row of 32000 with the rest of the GPU idle.)
+static __device__ __forceinline__ void run_argmax(const Stage& st, int tid) {
+  const int step = *st.step_counter;
+  __syncwarp();
+  if (tid < st.B) {
+    const unsigned long long key = __ldcg(st.best + tid);
+    st.best[tid] = 0ull;
+    const int bi = key ? (int)~(uint32_t)key : 0;
+    st.tokens[tid] = bi;
+    if (st.token_log && step < st.max_steps) st.token_log[(size_t)step * st.B + tid] = bi;
+    if (st.seqlens_rw) st.seqlens_rw[tid] += 1;
   }
   if (tid == 0) *st.step_counter = step + 1;
 }
@@ -1574,7 +1566,7 @@ fsvd_decode_kernel(const Stage* __restrict__ prog_global, const __grid_constant_
           if (st.type == ST_EMBED) {
             run_embed<T>(st, blockIdx.x * kConsThreads + tid, gridDim.x * kConsThreads);
           } else if (st.type == ST_ARGMAX) {
-            if (blockIdx.x == 0) run_argmax(st, red, flags_sh + 8, tid, kConsThreads);
+            if (blockIdx.x == 0 && warp == 0) run_argmax(st, tid);
           }
         }
       }

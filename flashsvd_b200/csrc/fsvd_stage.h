@@ -102,7 +102,7 @@ struct alignas(16) Stage {
   int* step_counter;     // incremented once per ST_ARGMAX
   int* seqlens_rw;       // [B] incremented by ST_ARGMAX
   int vocab, max_steps;
-  int reserved3[2];
+  unsigned long long* best;   // [B] running argmax keys: written by the lm_head stage (else null), read and zeroed by ST_ARGMAX
 };
 static_assert(sizeof(Stage) == 288, "Stage has no implicit padding");
 
