@@ -257,15 +257,16 @@ __global__ void __launch_bounds__(kThreads, 3) tile_gemm_kernel(const __grid_con
   const int p = tile * kTileM + r;           // factor row
   const int sl0 = 4 * (rope ? tid >> 6 : tid >> 7), sl_step = rope ? 16 : 8;
   const bool work = p < a.P;
+  const int B = min(a.B, bcol + a.N);        // end of this CTA's columns (slices are rounded up: the last one may end past it)
   // Operands of four columns that do not depend on the accumulators: residual elements, or the
   // position and the rotary pair.  Those of the first four are requested before the accumulators are
   // complete, those of the next four before the arithmetic of the four at hand.
   auto operands = [&](int sl, uint32_t (&x)[4], int (&pos)[4]) {
     const int b0 = bcol + seg * cpo + sl;
-    if (!work || sl >= cpo || b0 >= a.B) return;
+    if (!work || sl >= cpo || b0 >= B) return;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const int b = min(b0 + i, a.B - 1);
+      const int b = min(b0 + i, B - 1);
       if (a.epi == TE_RESID) {
         x[i] = reinterpret_cast<const unsigned short*>(a.resid)[(size_t)b * a.P + p];
       } else {
@@ -278,7 +279,7 @@ __global__ void __launch_bounds__(kThreads, 3) tile_gemm_kernel(const __grid_con
       }
     }
   };
-  const int epi = a.epi, segs = a.segs, B = a.B, P = a.P;   // (indexed constant loads: once, not per column)
+  const int epi = a.epi, segs = a.segs, P = a.P;   // (indexed constant loads: once, not per column)
   const bool two = a.two != 0;
   void* const out = a.out;
   const bool has_operands = rope || a.epi == TE_RESID || a.epi == TE_VCACHE;

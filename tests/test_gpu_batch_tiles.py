@@ -91,11 +91,12 @@ def test_decode_layer_tiles_ragged_ranks(dev):
     assert rel_linf(out, ref) <= TOL
 
 
-@pytest.mark.parametrize("B", [64, 65, 81, 127])
-def test_decode_layer_tiles_wide_batches_in_halves(dev, B):
+@pytest.mark.parametrize("B,I", [(64, 392), (65, 392), (81, 392), (127, 392), (66, 1544), (128, 1544), (128, 2072)])
+def test_decode_layer_tiles_wide_batches_in_halves(dev, B, I):
     """From 65 sequences on two CTAs take half of a tile's columns each (48 + 17, 48 + 33, 64 + 63 here, and
-    64 in one piece) and a CTA's column slice ends inside a group of four."""
-    shape = O.Shape(d=256, H=4, Hk=2, Dh=64, I=392, Rq=72, Rk=40, Rv=24, Ro=88, Rg=56, Ru=56, Rd=104, vocab=300, n_layers=1)
+    64 in one piece).  The longer products are cut into 5 and 7 K segments: slices of 16 and 12 columns, the
+    last of which end past the half's columns."""
+    shape = O.Shape(d=256, H=4, Hk=2, Dh=64, I=I, Rq=72, Rk=40, Rv=24, Ro=88, Rg=56, Ru=56, Rd=104, vocab=300, n_layers=1)
     out, ref, pk, kc_o, vc_o = _layer_case(dev, shape, B, 19, S_max=24)
     assert rel_linf(pk["k_cache"], kc_o) <= TOL
     assert rel_linf(pk["v_cache"], vc_o) <= TOL
