@@ -1078,8 +1078,17 @@ int fsvd_flash_decode(const void* q, const void* k_cache, const void* v_cache,
   if (int e = check_ws(D, ws, ws_bytes, L)) return e;
   Resolved r;
   if (int e = resolve(dtype, B, r)) return e;
-  Builder b(r, dtype, B);
   char* w = reinterpret_cast<char*>(ws);
+  if (!(scale > 0.f)) scale = 1.0f / sqrtf((float)Dh);
+  // bf16: the attention kernels of the tiled path, which read a cache row once for all the heads that
+  // share it and take as many key splits as fill the GPU (the interpreter's stage reads it once per two
+  // heads and takes at most 28: 8 kv heads x 64 heads x 2 sequences x 4096 keys 46 us).  They load 16 bytes
+  // at a time; other dtypes and pointers stay on the stage.
+  if (dtype != FSVD_DTYPE_F32 && aligned16(q) && aligned16(k_cache) && aligned16(v_cache) && aligned16(out))
+    return fsvd_tile_flash_decode(q, k_cache, v_cache, cache_seqlens, seqlen_add, out, B, H, Hk, Dh, S_max, scale,
+                                  reinterpret_cast<float*>(w + L.part_acc), (L.total - L.part_acc) / sizeof(float),
+                                  reinterpret_cast<int*>(w + L.counters), stream);
+  Builder b(r, dtype, B);
   Stage s = b.blank();
   s.type = ST_ATTN;
   s.flags = SF_IN_T | SF_OUT_T;
@@ -1093,7 +1102,7 @@ int fsvd_flash_decode(const void* q, const void* k_cache, const void* v_cache,
   s.part_ml = reinterpret_cast<float*>(w + L.part_ml);
   s.counters = reinterpret_cast<int*>(w + L.counters);
   s.H = H; s.Hk = Hk; s.Dh = Dh; s.S_max = S_max;
-  s.scale = scale > 0.f ? scale : 1.0f / sqrtf((float)Dh);
+  s.scale = scale;
   b.attn_geometry(s);
   b.push(s);
   return launch_small(r, b, reinterpret_cast<SyncState*>(w + L.sync), (cudaStream_t)stream);

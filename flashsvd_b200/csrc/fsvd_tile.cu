@@ -44,6 +44,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <atomic>
 #include <initializer_list>
 #include <mutex>
 #include <utility>
@@ -672,6 +673,12 @@ struct AttnArgs {
   float scale;
 };
 
+// FULL: the op on its own (fsvd_flash_decode) keeps softmax weights in 32 bits: expf, and on the tensor
+// cores each weight as the sum of two bf16 numbers (16 significant bits; the value rows are bf16 and the
+// result is rounded to bf16).  Inside a model step the weights are bf16 where they meet the tensor cores.
+template <bool FULL>
+__device__ __forceinline__ float weight(float x) { return FULL ? expf(x) : __expf(x); }
+
 template <int DPL>
 __device__ __forceinline__ void ld_row(const __nv_bfloat16* row, int lane, float (&f)[DPL]);
 template <>
@@ -686,7 +693,7 @@ __device__ __forceinline__ void ld_row<2>(const __nv_bfloat16* row, int lane, fl
   f[0] = __uint_as_float(w << 16); f[1] = __uint_as_float(w & 0xffff0000u);
 }
 
-template <int DH, int G>
+template <int DH, int G, bool FULL>
 __global__ void __launch_bounds__(kAttnThreads) batch_attn_kernel(const AttnArgs a) {
   constexpr int DPL = DH / 32;
   __shared__ float wm[kAttnWarps][G], wl[kAttnWarps][G];
@@ -751,14 +758,14 @@ __global__ void __launch_bounds__(kAttnThreads) batch_attn_kernel(const AttnArgs
         cm = fmaxf(cm, s[i]);
       }
       const float mn = fmaxf(m[g], cm);
-      const float corr = __expf(m[g] - mn);                 // 0 when m is still -inf
+      const float corr = weight<FULL>(m[g] - mn);                 // 0 when m is still -inf
       m[g] = mn;
       float ps = 0.0f;
 #pragma unroll
       for (int e = 0; e < DPL; ++e) acc[g][e] *= corr;
 #pragma unroll
       for (int i = 0; i < kKeyGroup; ++i) {
-        const float pr = __expf(s[i] - mn);               // 0 for the masked rows
+        const float pr = weight<FULL>(s[i] - mn);               // 0 for the masked rows
         ps += pr;
 #pragma unroll
         for (int e = 0; e < DPL; ++e) acc[g][e] += pr * vf[i][e];
@@ -788,7 +795,7 @@ __global__ void __launch_bounds__(kAttnThreads) batch_attn_kernel(const AttnArgs
     float num = 0.0f, den = 0.0f;
 #pragma unroll
     for (int w = 0; w < kAttnWarps; ++w) {
-      const float wgt = wm[w][g] == -INFINITY ? 0.0f : __expf(wm[w][g] - mm);
+      const float wgt = wm[w][g] == -INFINITY ? 0.0f : weight<FULL>(wm[w][g] - mm);
       num += wgt * wacc[w][g][dd];
       den += wgt * wl[w][g];
     }
@@ -822,7 +829,7 @@ __global__ void __launch_bounds__(kAttnThreads) batch_attn_kernel(const AttnArgs
     for (int sp = 0; sp < nsplit; ++sp) {
       const float* pr = parts + ((size_t)sp * G + g) * rec;
       const float ms = __ldcg(pr + DH);
-      const float wgt = ms == -INFINITY ? 0.0f : __expf(ms - mm);
+      const float wgt = ms == -INFINITY ? 0.0f : weight<FULL>(ms - mm);
       num += wgt * __ldcg(pr + dd);
       den += wgt * __ldcg(pr + DH + 1);
     }
@@ -842,7 +849,7 @@ __global__ void __launch_bounds__(kAttnThreads) batch_attn_kernel(const AttnArgs
 constexpr int kGqKeys = 32;      // keys per warp block
 constexpr int kGqMaxSplit = 64;  // key splits of a sequence at most
 
-template <int DH>
+template <int DH, bool FULL>
 __global__ void __launch_bounds__(kAttnThreads, 3) gqa_decode_attn_kernel(const AttnArgs a) {
   constexpr int STRIDE = DH * 2 + 16;
   constexpr int KS = DH / 16, NT = kGqKeys / 8, DT = DH / 8;
@@ -924,14 +931,14 @@ __global__ void __launch_bounds__(kAttnThreads, 3) gqa_decode_attn_kernel(const 
     mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
     mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
     const float mn = fmaxf(mrow, mx);           // finite: key k0 is inside the split
-    const float corr = __expf(mrow - mn);
+    const float corr = weight<FULL>(mrow - mn);
     mrow = mn;
     float ps = 0.0f;
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) {
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        const float pr = __expf(sc[nt][e] - mn);
+        const float pr = weight<FULL>(sc[nt][e] - mn);
         sc[nt][e] = pr;
         ps += pr;
       }
@@ -949,6 +956,11 @@ __global__ void __launch_bounds__(kAttnThreads, 3) gqa_decode_attn_kernel(const 
     for (int kk = 0; kk < kGqKeys / 16; ++kk) {
       const uint32_t pa0 = pack_bf16(sc[2 * kk][0], sc[2 * kk][1]);
       const uint32_t pa2 = pack_bf16(sc[2 * kk + 1][0], sc[2 * kk + 1][1]);
+      uint32_t pl0 = 0u, pl2 = 0u;
+      if (FULL) {
+        pl0 = pack_bf16(sc[2 * kk][0] - rnd(sc[2 * kk][0]), sc[2 * kk][1] - rnd(sc[2 * kk][1]));
+        pl2 = pack_bf16(sc[2 * kk + 1][0] - rnd(sc[2 * kk + 1][0]), sc[2 * kk + 1][1] - rnd(sc[2 * kk + 1][1]));
+      }
       const int lr = kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8;
       const unsigned char* vr = vs_s + lr * STRIDE + ((lane >> 4) & 1) * 16;
 #pragma unroll
@@ -960,6 +972,10 @@ __global__ void __launch_bounds__(kAttnThreads, 3) gqa_decode_attn_kernel(const 
         float c0[4] = {o[2 * j][0], o[2 * j][1], 0.0f, 0.0f}, c1[4] = {o[2 * j + 1][0], o[2 * j + 1][1], 0.0f, 0.0f};
         mma_bf16_16816(c0, pa0, 0u, pa2, 0u, b0, b1);
         mma_bf16_16816(c1, pa0, 0u, pa2, 0u, b2, b3);
+        if (FULL) {
+          mma_bf16_16816(c0, pl0, 0u, pl2, 0u, b0, b1);
+          mma_bf16_16816(c1, pl0, 0u, pl2, 0u, b2, b3);
+        }
         o[2 * j][0] = c0[0]; o[2 * j][1] = c0[1];
         o[2 * j + 1][0] = c1[0]; o[2 * j + 1][1] = c1[1];
       }
@@ -995,7 +1011,7 @@ __global__ void __launch_bounds__(kAttnThreads, 3) gqa_decode_attn_kernel(const 
 #pragma unroll
     for (int w = 0; w < kAttnWarps; ++w) {
       const float* pr = wpart + ((size_t)w * G + gg) * rec;
-      const float wgt = pr[DH] == -INFINITY ? 0.0f : __expf(pr[DH] - mm);
+      const float wgt = pr[DH] == -INFINITY ? 0.0f : weight<FULL>(pr[DH] - mm);
       num += wgt * pr[dd];
       den += wgt * pr[DH + 1];
     }
@@ -1040,7 +1056,7 @@ __global__ void __launch_bounds__(kAttnThreads, 3) gqa_decode_attn_kernel(const 
   __syncthreads();
   for (int i = tid; i < nsplit * G; i += kAttnThreads) {
     const float ms = wgt_s[i];
-    wgt_s[i] = ms == -INFINITY ? 0.0f : __expf(ms - den_s[8 + i % G]);
+    wgt_s[i] = ms == -INFINITY ? 0.0f : weight<FULL>(ms - den_s[8 + i % G]);
   }
   __syncthreads();
   if (tid < G) {
@@ -1401,20 +1417,25 @@ struct TileWs {
   size_t sync, counters, xn, pbuf, qbuf, attn, mid, hact, apart, total;
   int nsplit;
 };
-static int attn_nsplit(const fsvd_dims& D, int sms) {
-  if (D.rows_are_positions) return 1;   // prompt pass: row blocks share the cache rows instead
-  if (D.Hk > 0 && D.H / D.Hk >= 4) {
+// Key splits of a sequence.  pairs = sequences x kv heads, positions = longest sequence the cache holds.
+static int attn_splits(int pairs, int G, int positions, int sms, int most) {
+  if (G >= 4) {
     // grouped-query kernel: 3 CTAs per SM, at least one block of 32 keys for each of a CTA's 4 warps
-    int ns = (3 * sms + D.B * D.Hk - 1) / (D.B * D.Hk);
-    const int most = (D.S_max + 4 * kGqKeys - 1) / (4 * kGqKeys);
-    if (ns > most) ns = most;
-    if (ns > kGqMaxSplit) ns = kGqMaxSplit;
-    return ns < 1 ? 1 : ns;
+    most = std::min(most, (positions + 4 * kGqKeys - 1) / (4 * kGqKeys));
+    return std::max(1, std::min((3 * sms + pairs - 1) / pairs, most));
   }
-  int ns = (8 * sms + D.B * D.Hk - 1) / (D.B * D.Hk);   // about 8 CTAs of 4 warps per SM
-  if (ns > 16) ns = 16;
-  if (ns < 1) ns = 1;
-  return ns;
+  // Three waves of the 8 CTAs of 4 warps that an SM holds, so that the SMs even out: not more than 8 splits
+  // for that, the merge grows with them, but as many as one wave takes.  Measured, 4 layers, 4 steps (us):
+  // 8 sequences x 32 heads x 2048 keys 5 splits 2659, 8 2588, 16 2636; 32 sequences 2 splits 4999, 4 4862, 8
+  // 4872; 128 sequences x 640 keys 1 split 6494, 2 6658.
+  most = std::max(1, std::min(most, (positions + kAttnWarps * kKeyGroup - 1) / (kAttnWarps * kKeyGroup)));
+  const int wave = (8 * sms + pairs - 1) / pairs;
+  return std::min(most, std::min((24 * sms + pairs - 1) / pairs, std::max(8, wave)));
+}
+static int attn_nsplit(const fsvd_dims& D, int sms) {
+  if (D.rows_are_positions || D.Hk < 1) return 1;   // prompt pass: row blocks share the cache rows instead
+  const int G = D.H / D.Hk;
+  return attn_splits(D.B * D.Hk, G, D.S_max, sms, G >= 4 ? kGqMaxSplit : 16);
 }
 static int imax(int a, int b) { return a > b ? a : b; }
 static TileWs tile_layout(const fsvd_dims& D, int sms) {
@@ -1567,23 +1588,25 @@ static void launch_prompt_attn(const PaArgs& pa, int Dh, int nseq, cudaStream_t 
   fsvd_tile_count_launch();
 }
 
-template <int DH>
+template <int DH, bool FULL>
 static void launch_attn_g(const AttnArgs& at, cudaStream_t st) {
   const unsigned threads = kAttnThreads;
   const int G = at.H / at.Hk;
   const unsigned grid = (unsigned)(at.B * at.Hk * at.nsplit);
   switch (G) {
-    case 1: launch_pdl(batch_attn_kernel<DH, 1>, dim3(grid), dim3(threads), 0, st, at); break;
-    case 2: launch_pdl(batch_attn_kernel<DH, 2>, dim3(grid), dim3(threads), 0, st, at); break;
+    case 1: launch_pdl(batch_attn_kernel<DH, 1, FULL>, dim3(grid), dim3(threads), 0, st, at); break;
+    case 2: launch_pdl(batch_attn_kernel<DH, 2, FULL>, dim3(grid), dim3(threads), 0, st, at); break;
     default: {
       // 4 or 8 heads per kv head: the heads as rows of a tensor-core tile
       constexpr size_t smem = (size_t)kAttnWarps * 2 * kGqKeys * (DH * 2 + 16);
-      static bool attr_set = false;   // per instantiation; set under the planner's lock or at first use
-      if (!attr_set) {
-        cudaFuncSetAttribute(gqa_decode_attn_kernel<DH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        attr_set = true;
+      static std::atomic<unsigned long long> attr_set{0};   // per instantiation: a bit per device
+      int dev = 0;
+      cudaGetDevice(&dev);
+      if (dev > 63 || !(attr_set.load(std::memory_order_relaxed) >> dev & 1)) {
+        cudaFuncSetAttribute(gqa_decode_attn_kernel<DH, FULL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (dev <= 63) attr_set.fetch_or(1ull << dev);
       }
-      launch_pdl(gqa_decode_attn_kernel<DH>, dim3(grid), dim3(threads), smem, st, at);
+      launch_pdl(gqa_decode_attn_kernel<DH, FULL>, dim3(grid), dim3(threads), smem, st, at);
     }
   }
 }
@@ -1594,15 +1617,15 @@ static PaArgs prompt_args(const AttnArgs& at) {
   pa.scale_log2 = at.scale * 1.4426950408889634f;
   return pa;
 }
-static int launch_attn(const AttnArgs& at, cudaStream_t st) {
+static int launch_attn(const AttnArgs& at, cudaStream_t st, bool full = false) {
   if (at.shared_cache) {
     // the rows are consecutive positions of one sequence
     launch_prompt_attn(prompt_args(at), at.Dh, 1, st);
     if (cudaGetLastError() != cudaSuccess) return fail(FSVD_ERR_CUDA, "attention kernel launch failed");
     return 0;
   }
-  if (at.Dh == 128) launch_attn_g<128>(at, st);
-  else launch_attn_g<64>(at, st);
+  if (at.Dh == 128) full ? launch_attn_g<128, true>(at, st) : launch_attn_g<128, false>(at, st);
+  else full ? launch_attn_g<64, true>(at, st) : launch_attn_g<64, false>(at, st);
   if (cudaGetLastError() != cudaSuccess) return fail(FSVD_ERR_CUDA, "attention kernel launch failed");
   fsvd_tile_count_launch();
   return 0;
@@ -1714,6 +1737,24 @@ static int plan_tp_layer(TpPlan& tp, const fsvd_dims& D, const fsvd_layer& Lw, c
 
 // ------------------------------------------------------------------------------- entry points
 using namespace fsvd_tile;
+
+int fsvd_tile_flash_decode(const void* q, const void* k_cache, const void* v_cache, const int* cache_seqlens, int seqlen_add,
+                           void* out, int B, int H, int Hk, int Dh, int S_max, float scale, float* part, size_t part_floats,
+                           int* counters, void* stream) {
+  if (int e = device_limits()) return e;
+  AttnArgs at;
+  memset(&at, 0, sizeof(at));
+  at.q = reinterpret_cast<const __nv_bfloat16*>(q);
+  at.kcache = reinterpret_cast<const __nv_bfloat16*>(k_cache);
+  at.vcache = reinterpret_cast<const __nv_bfloat16*>(v_cache);
+  at.seqlens = cache_seqlens; at.out = reinterpret_cast<__nv_bfloat16*>(out);
+  at.part = part; at.counters = counters;
+  at.B = B; at.H = H; at.Hk = Hk; at.Dh = Dh; at.S_max = S_max; at.seqlen_add = seqlen_add; at.scale = scale;
+  // a split's record is Dh + 4 floats per head at most
+  const int fits = (int)std::min<size_t>(part_floats / ((size_t)B * H * (Dh + 4)), kGqMaxSplit);
+  at.nsplit = attn_splits(B * Hk, H / Hk, S_max, g_sms, std::max(1, fits));
+  return launch_attn(at, (cudaStream_t)stream, true);
+}
 
 size_t fsvd_tile_workspace_bytes(const fsvd_dims* dims) {
   if (!dims || device_limits()) return 0;

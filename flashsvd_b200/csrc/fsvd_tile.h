@@ -28,6 +28,10 @@ int fsvd_tile_model_create(const fsvd_dims* dims, const fsvd_layer* layers, cons
                            const void* lm_head, const void* cos_tab, const void* sin_tab, int max_steps, long long wait_limit,
                            fsvd_tile_model** out);
 int fsvd_tile_model_destroy(fsvd_tile_model* m);
+// Single-query attention on its own (bf16): `part` / `counters` as in the model step, counters zero between calls.
+int fsvd_tile_flash_decode(const void* q, const void* k_cache, const void* v_cache, const int* cache_seqlens, int seqlen_add,
+                           void* out, int B, int H, int Hk, int Dh, int S_max, float scale, float* part, size_t part_floats,
+                           int* counters, void* stream);
 int fsvd_tile_model_step(fsvd_tile_model* m, int n_steps, void* stream);
 void fsvd_tile_model_buffers(fsvd_tile_model* m, int** tokens, int** seqlens, int** token_log, int** step_counter,
                              float** logits, float** hidden);
