@@ -1427,8 +1427,9 @@ static int attn_splits(int pairs, int G, int positions, int sms, int most) {
   // Three waves of the 8 CTAs of 4 warps that an SM holds, so that the SMs even out: not more than 8 splits
   // for that, the merge grows with them, but as many as one wave takes.  Measured, 4 layers, 4 steps (us):
   // 8 sequences x 32 heads x 2048 keys 5 splits 2659, 8 2588, 16 2636; 32 sequences 2 splits 4999, 4 4862, 8
-  // 4872; 128 sequences x 640 keys 1 split 6494, 2 6658.
-  most = std::max(1, std::min(most, (positions + kAttnWarps * kKeyGroup - 1) / (kAttnWarps * kKeyGroup)));
+  // 4872; 128 sequences x 640 keys 1 split 6494, 2 6658.  A split gets two groups of keys per warp: attention
+  // half with 2 heads per kv head, 8 sequences, 300 keys 78 us with one, 74 with two.
+  most = std::max(1, std::min(most, (positions + 2 * kAttnWarps * kKeyGroup - 1) / (2 * kAttnWarps * kKeyGroup)));
   const int wave = (8 * sms + pairs - 1) / pairs;
   return std::min(most, std::min((24 * sms + pairs - 1) / pairs, std::max(8, wave)));
 }
