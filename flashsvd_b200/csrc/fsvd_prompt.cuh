@@ -16,7 +16,8 @@
 
 namespace fsvd_tile {
 
-constexpr int kPgThreads = 192;      // warp 0 producer, warp 1 MMA, warps 2..5 epilogue
+constexpr int kPgThreads = 256;      // warp 1 MMA, warps 2..5 epilogue, warps 0, 6, 7 producers
+constexpr int kPgProducers = 3;
 constexpr int kPgMaxStages = 8;
 constexpr int kPgBufCols = 256;      // tensor-memory columns of an accumulator buffer (two buffers)
 constexpr int kPgBoxRows = 64;       // factor rows of a TMA box
@@ -132,8 +133,9 @@ __global__ void __launch_bounds__(kPgThreads, 1) prompt_gemm_kernel(const __grid
   pdl_launch_dependents();
   pdl_wait();
 
-  if (warp == 0) {
+  if (warp == 0 || warp >= 6) {
     if (lane == 0) {
+      const int pj = warp == 0 ? 0 : warp - 5;
       int s = 0, round = 0;
       bool ok = true;
       for (int tile = blockIdx.x; tile < a.total && ok; tile += gridDim.x) {
@@ -142,6 +144,13 @@ __global__ void __launch_bounds__(kPgThreads, 1) prompt_gemm_kernel(const __grid
         const uint32_t wbytes = (uint32_t)pr.nt * 128u;
         const uint32_t bytes = (kTileM * 128u + wbytes) * (pr.two ? 2u : 1u);
         for (int kb = 0; kb < pr.nkb; ++kb) {
+          if (s % kPgProducers != pj) {   // another producer's slot
+            if (++s == NS) {
+              s = 0;
+              ++round;
+            }
+            continue;
+          }
           if (round > 0 && !(ok = wait_bar(empty0 + 8 * s, (uint32_t)(round - 1) & 1u, giveup, a.status, a.wait_limit, DS_COPY_TIMEOUT))) break;
           const uint32_t fb = full0 + 8 * s;
           uint32_t dst = base + (uint32_t)s * (uint32_t)a.stage_bytes;
