@@ -1123,6 +1123,8 @@ int fsvd_decode_layer(const fsvd_dims* dims, const fsvd_layer* layer, const void
   }
   if (int e = check_dims(D)) return e;
   if (int e = check_layer_ptrs(*layer)) return e;
+  // (the single-launch kernel reads the hidden state 16 bytes at a time; the tiled path takes any address)
+  if (!aligned16(x_in)) return fail(FSVD_ERR_ALIGN, "x_in must be 16-byte aligned for batches of the single-launch kernel");
   WsLayout L;
   if (int e = check_ws(D, ws, ws_bytes, L)) return e;
   Resolved r;

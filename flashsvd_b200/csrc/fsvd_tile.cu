@@ -439,6 +439,15 @@ __global__ void __launch_bounds__(kThreads, 3) tile_gemm_kernel(const __grid_con
 // ------------------------------------------------------------------------------- RMSNorm rows
 // out[b, :] = rnd(w * rnd(x[r, :] * rsqrt(mean(x[r, :]^2) + eps))), r = b * row_mul + row_off, one CTA per
 // row.  A thread's 16-byte pieces stay in registers between the two passes (rows up to 8192 wide).
+// WIDE: x starts on a 16-byte boundary; a caller's hidden state that does not is read 2 bytes at a time
+// (w and out always do: layer pointers are checked, out is the library's own).
+template <bool WIDE>
+__device__ __forceinline__ uint4 load_8bf(const __nv_bfloat16* p) {
+  if (WIDE) return *reinterpret_cast<const uint4*>(p);
+  const unsigned short* h = reinterpret_cast<const unsigned short*>(p);
+  return make_uint4(h[0] | (uint32_t)h[1] << 16, h[2] | (uint32_t)h[3] << 16, h[4] | (uint32_t)h[5] << 16, h[6] | (uint32_t)h[7] << 16);
+}
+template <bool WIDE>
 __global__ void __launch_bounds__(256) rmsnorm_rows_kernel(const __nv_bfloat16* __restrict__ x,
                                                            const __nv_bfloat16* __restrict__ w,
                                                            __nv_bfloat16* __restrict__ out, int d, float eps,
@@ -448,7 +457,7 @@ __global__ void __launch_bounds__(256) rmsnorm_rows_kernel(const __nv_bfloat16* 
   const int b = blockIdx.x, tid = threadIdx.x, n8 = d >> 3;
   pdl_launch_dependents();
   pdl_wait();
-  const uint4* xr = reinterpret_cast<const uint4*>(x + (size_t)(b * row_mul + row_off) * d);
+  const __nv_bfloat16* xr = x + (size_t)(b * row_mul + row_off) * d;
   const uint4* wr = reinterpret_cast<const uint4*>(w);
   uint4* orow = reinterpret_cast<uint4*>(out + (size_t)b * d);
   const bool fits = n8 <= 256 * U;
@@ -458,7 +467,7 @@ __global__ void __launch_bounds__(256) rmsnorm_rows_kernel(const __nv_bfloat16* 
 #pragma unroll
     for (int k = 0; k < U; ++k)
       if (i0 + 256 * k < n8) {
-        v[k] = xr[i0 + 256 * k];
+        v[k] = load_8bf<WIDE>(xr + 8 * (i0 + 256 * k));
         wv[k] = wr[i0 + 256 * k];
       }
 #pragma unroll
@@ -495,7 +504,7 @@ __global__ void __launch_bounds__(256) rmsnorm_rows_kernel(const __nv_bfloat16* 
     for (int k = 0; k < U; ++k)
       if (tid + 256 * k < n8) finish(tid + 256 * k, v[k], wv[k]);
   } else {
-    for (int i = tid; i < n8; i += 256) finish(i, xr[i], wr[i]);
+    for (int i = tid; i < n8; i += 256) finish(i, load_8bf<WIDE>(xr + 8 * i), wr[i]);
   }
 }
 
@@ -1652,8 +1661,8 @@ static int run_layer(const LayerPlan& lp, const GemmPlan& down_lift, const fsvd_
   const __nv_bfloat16* mid = reinterpret_cast<const __nv_bfloat16*>(ws + L.mid);
   int e;
   if (!have_xn) {
-    launch_pdl(rmsnorm_rows_kernel, dim3(D.B), dim3(256), 0, st, reinterpret_cast<const __nv_bfloat16*>(x_in),
-               reinterpret_cast<const __nv_bfloat16*>(Lw.ln1_w), xn, D.d, D.eps, 1, 0);
+    launch_pdl(reinterpret_cast<uintptr_t>(x_in) % 16 ? rmsnorm_rows_kernel<false> : rmsnorm_rows_kernel<true>, dim3(D.B), dim3(256), 0,
+               st, reinterpret_cast<const __nv_bfloat16*>(x_in), reinterpret_cast<const __nv_bfloat16*>(Lw.ln1_w), xn, D.d, D.eps, 1, 0);
     fsvd_tile_count_launch();
   }
   if ((e = launch_gemm(lp.g[0], st))) return e;
@@ -1672,7 +1681,7 @@ static int run_layer(const LayerPlan& lp, const GemmPlan& down_lift, const fsvd_
   if (r1) {
     if ((e = launch_reduce(*r1, D.B, st))) return e;
   } else {
-    launch_pdl(rmsnorm_rows_kernel, dim3(D.B), dim3(256), 0, st, mid, reinterpret_cast<const __nv_bfloat16*>(Lw.ln2_w), xn,
+    launch_pdl(rmsnorm_rows_kernel<true>, dim3(D.B), dim3(256), 0, st, mid, reinterpret_cast<const __nv_bfloat16*>(Lw.ln2_w), xn,
                D.d, D.eps, 1, 0);
     fsvd_tile_count_launch();
   }
@@ -1900,7 +1909,7 @@ static int tile_model_record(fsvd_tile_model* m, cudaStream_t st) {
   for (int l = 0; l < D.n_layers; ++l)
     if ((e = run_layer(m->layers[l], m->down[l], D, m->lw[l], m->xbuf[l & 1], m->ws, m->L, st))) return e;
   __nv_bfloat16* xn = reinterpret_cast<__nv_bfloat16*>(m->ws + m->L.xn);
-  launch_pdl(rmsnorm_rows_kernel, dim3(D.B), dim3(256), 0, st, (const __nv_bfloat16*)m->xbuf[D.n_layers & 1],
+  launch_pdl(rmsnorm_rows_kernel<true>, dim3(D.B), dim3(256), 0, st, (const __nv_bfloat16*)m->xbuf[D.n_layers & 1],
              reinterpret_cast<const __nv_bfloat16*>(m->final_norm), xn, D.d, D.eps, 1, 0);
   fsvd_tile_count_launch();
   if ((e = launch_gemm(m->head, st))) return e;
@@ -2233,7 +2242,7 @@ int fsvd_tile_prompt_run(fsvd_tile_prompt* p, const int* prompt, int ld, int L, 
   if (int e = prompt_reserve(p, len * D.B)) return e;
   const int HD = D.H * D.Dh, KD = D.Hk * D.Dh, Rqkv = D.Rq + D.Rk + D.Rv;
   auto norm = [&](const __nv_bfloat16* x, const void* w, __nv_bfloat16* out, int rows, int mul, int off) {
-    launch_pdl(rmsnorm_rows_kernel, dim3((unsigned)rows), dim3(256), 0, st, x, reinterpret_cast<const __nv_bfloat16*>(w), out, D.d, D.eps,
+    launch_pdl(rmsnorm_rows_kernel<true>, dim3((unsigned)rows), dim3(256), 0, st, x, reinterpret_cast<const __nv_bfloat16*>(w), out, D.d, D.eps,
                mul, off);
     fsvd_tile_count_launch();
   };

@@ -103,6 +103,44 @@ def test_decode_layer_tiles_wide_batches_in_halves(dev, B, I):
     assert rel_linf(out, ref) <= TOL
 
 
+@pytest.mark.parametrize("B", [5, 17, 2])
+@pytest.mark.parametrize("d", [264, 8200])
+def test_decode_layer_hidden_state_at_any_address(dev, B, d):
+    """A contiguous hidden state that does not start on a 16-byte boundary: the tiled path (5 sequences on)
+    reads it 2 bytes at a time, with the same result bit for bit (rows within and beyond what the norm keeps
+    in registers); the single-launch kernel refuses it before a launch."""
+    from flashsvd_b200 import ops, packing
+
+    shape = O.Shape(d=d, H=4, Hk=2, Dh=64, I=72, Rq=24, Rk=16, Rv=16, Ro=24, Rg=24, Ru=24, Rd=24, vocab=200, n_layers=1)
+    dtype, S_max = torch.bfloat16, 16
+    gen = torch.Generator().manual_seed(d + B)
+    w = O.make_layer_weights(shape, gen, dtype)
+    x = torch.randn(B, d, generator=gen).to(dtype)
+    cos, sin = (t.to(dev) for t in O.rope_tables(S_max, shape.Dh, shape.theta, dtype))
+    pk = packing.pack_layer(w, device=dev, dtype=dtype)
+    dims = ops.make_dims(dtype=dtype, B=B, d=d, H=4, Hk=2, Dh=64, I=72, Rq=24, Rk=16, Rv=16, Ro=24, Rg=24, Ru=24, Rd=24,
+                         S_max=S_max, eps=shape.eps)
+    ws = ops.make_workspace(dims, dev)
+    lens = torch.arange(B, dtype=torch.int32, device=dev) % 4
+    results = []
+    for offset in (0, 1, 4):   # elements past an aligned address
+        buf = torch.empty(B * d + offset, dtype=dtype, device=dev)
+        xd = buf[offset:].view(B, d)
+        xd.copy_(x)
+        pk["k_cache"], pk["v_cache"] = (torch.zeros(B, S_max, 2, 64, dtype=dtype, device=dev) for _ in range(2))
+        out = torch.empty(B, d, dtype=dtype, device=dev)
+        call = lambda: ops.decode_layer(dims, ops.make_layer_struct(pk), cos, sin, lens, xd, out, ws)
+        if offset and B < 5:
+            with pytest.raises(ValueError, match="x_in"):
+                call()
+            continue
+        call()
+        assert ws.status() == 0
+        results.append((out, pk["k_cache"], pk["v_cache"]))
+    for r in results[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(r, results[0]))
+
+
 @pytest.mark.parametrize("B", [16, 32])
 def test_decode_layer_tiles_7b_shape(dev, B):
     # one Llama-2-7B-shaped layer, ranks 1024 / 1488, 512 cached positions
