@@ -1934,6 +1934,19 @@ int fsvd_tile_model_destroy(fsvd_tile_model* m) {
   return 0;
 }
 
+// Zeroes fresh device memory before any stream can use it.  (cudaMemset goes to the default stream and returns
+// at once; a pass on a non-blocking stream would not wait for it.  A stream of its own does not wait for
+// what the default stream has queued.)
+static cudaError_t clear_now(void* p, size_t bytes) {
+  cudaStream_t st;
+  cudaError_t ce = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+  if (ce != cudaSuccess) return ce;
+  ce = cudaMemsetAsync(p, 0, bytes, st);
+  if (ce == cudaSuccess) ce = cudaStreamSynchronize(st);
+  cudaStreamDestroy(st);
+  return ce;
+}
+
 int fsvd_tile_model_create(const fsvd_dims* dims, const fsvd_layer* layers, const void* embed, const void* final_norm_w,
                            const void* lm_head, const void* cos_tab, const void* sin_tab, int max_steps, long long wait_limit,
                            fsvd_tile_model** out) {
@@ -1953,8 +1966,8 @@ int fsvd_tile_model_create(const fsvd_dims* dims, const fsvd_layer* layers, cons
   if (ce == cudaSuccess) ce = cudaMalloc(&m->extra, extra);
   if (ce == cudaSuccess) ce = cudaMalloc(&m->xbuf[0], al256((size_t)D.B * D.d * 2));
   if (ce == cudaSuccess) ce = cudaMalloc(&m->xbuf[1], al256((size_t)D.B * D.d * 2));
-  if (ce == cudaSuccess) ce = cudaMemset(m->ws, 0, m->L.total);
-  if (ce == cudaSuccess) ce = cudaMemset(m->extra, 0, extra);
+  if (ce == cudaSuccess) ce = clear_now(m->ws, m->L.total);
+  if (ce == cudaSuccess) ce = clear_now(m->extra, extra);
   if (ce != cudaSuccess) {
     fsvd_tile_model_destroy(m);
     return fail(FSVD_ERR_CUDA, "allocating model scratch failed");
@@ -2094,7 +2107,7 @@ int fsvd_tile_prompt_create(const fsvd_dims* dims, const fsvd_layer* layers, con
   p->wait_limit = wait_limit;
   const size_t fixed = al256(sizeof(SyncState)) + al256((size_t)D.B * D.d * 2);
   cudaError_t ce = cudaMalloc(&p->fixed, fixed);
-  if (ce == cudaSuccess) ce = cudaMemset(p->fixed, 0, fixed);
+  if (ce == cudaSuccess) ce = clear_now(p->fixed, fixed);
   if (ce == cudaSuccess)
     ce = cudaFuncSetAttribute(tile_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, g_smem_optin - 1024);
   if (ce == cudaSuccess)
@@ -2140,11 +2153,7 @@ static int prompt_reserve(fsvd_tile_prompt* p, int rows) {
   }
   char* ws = nullptr;
   if (cudaMalloc(&ws, total) != cudaSuccess) return fail(FSVD_ERR_CUDA, "allocating prompt scratch failed");
-  // rows past a pass's last one are multiplied too (and never stored): they have to be numbers the first time
-  if (cudaMemset(ws, 0, total) != cudaSuccess) {
-    cudaFree(ws);
-    return fail(FSVD_ERR_CUDA, "clearing prompt scratch failed");
-  }
+  // (not cleared: the rows past a pass's last one, multiplied too, reach only accumulator rows that are never stored)
   cudaFree(p->ws);   // (waits for the passes that still use it)
   p->ws = ws;
   p->cap = cap;

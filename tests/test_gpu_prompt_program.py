@@ -14,6 +14,20 @@ RAGGED = O.Shape(d=264, H=4, Hk=2, Dh=64, I=520, Rq=88, Rk=40, Rv=56, Ro=72, Rg=
 WIDE_HEADS = O.Shape(d=512, H=8, Hk=1, Dh=128, I=1096, Rq=136, Rk=64, Rv=64, Ro=128, Rg=200, Ru=200, Rd=192, vocab=300, n_layers=2)
 
 
+def _engine(shape, w, B, S_max, **over):
+    from flashsvd_b200 import engine, packing
+
+    dev, dtype = torch.device("cuda:0"), w["embed"].dtype
+    return engine.DecodeEngine(layers=[packing.pack_layer(lw, device=dev, dtype=dtype) for lw in w["layers"]],
+                               embed=w["embed"].to(dev), final_norm=w["norm"].to(dev), lm_head=w["lm_head"].to(dev),
+                               num_heads=shape.H, num_kv_heads=shape.Hk, head_dim=shape.Dh, batch_size=B, max_cache_len=S_max,
+                               rope_theta=shape.theta, eps=shape.eps, max_steps=S_max + 4, **over)
+
+
+def _state(eng):
+    return [t.clone() for t in (eng.logits, eng.tokens, eng.seqlens, *eng.key_cache, *eng.value_cache)]
+
+
 def rel_linf(a, b):
     a, b = a.float().cpu(), b.float().cpu()
     return float((a - b).abs().max() / b.abs().max().clamp_min(1e-30))
@@ -22,16 +36,11 @@ def rel_linf(a, b):
 @pytest.mark.parametrize("shape,B,parts", [(RAGGED, 3, (2,)), (RAGGED, 3, (43, 86)), (RAGGED, 1, (128, 1)), (RAGGED, 2, (65, 64)),
                                            (WIDE_HEADS, 5, (26, 3)), (O.TINY, 9, (29,)), (WIDE_HEADS, 1, (257,))])
 def test_prompts_in_parts_match_oracle(shape, B, parts):
-    from flashsvd_b200 import engine, packing
-
-    dev, dtype, L = torch.device("cuda:0"), torch.bfloat16, sum(parts)
+    dtype, L = torch.bfloat16, sum(parts)
     w = O.make_model_weights(shape, seed=3, dtype=dtype)
     prompt = torch.randint(0, shape.vocab, (B, L), generator=torch.Generator().manual_seed(L))
     toks_ref, logits_ref, st = O.greedy_decode(shape, w, prompt, 1, S_max=L + 4)
-    eng = engine.DecodeEngine(layers=[packing.pack_layer(lw, device=dev, dtype=dtype) for lw in w["layers"]],
-                              embed=w["embed"].to(dev), final_norm=w["norm"].to(dev), lm_head=w["lm_head"].to(dev),
-                              num_heads=shape.H, num_kv_heads=shape.Hk, head_dim=shape.Dh, batch_size=B,
-                              max_cache_len=L + 4, rope_theta=shape.theta, eps=shape.eps, max_steps=L + 8)
+    eng = _engine(shape, w, B, L + 4)
     t0 = 0
     for n in parts:
         eng.prefill(prompt[:, t0:t0 + n])
@@ -48,3 +57,37 @@ def test_prompts_in_parts_match_oracle(shape, B, parts):
         eng.prefill(prompt[:, :2].repeat(1, 5))    # past the end of the cache: refused before a launch
     assert eng.status() == 0
     eng.close()
+
+
+@pytest.mark.parametrize("B", [2, 12])
+def test_first_prompt_on_a_side_stream(B):
+    """The first prompt of an engine (its program and scratch are made by that call, and for 12 sequences the
+    decode model just before) on a stream that does not wait for the default stream, which is busy: the same
+    values as on an idle device, also after the default stream has run dry."""
+    shape, L = RAGGED, 90
+    w = O.make_model_weights(shape, seed=5, dtype=torch.bfloat16)
+    prompt = torch.randint(0, shape.vocab, (B, L), generator=torch.Generator().manual_seed(B), dtype=torch.int32).cuda()
+    ref = _engine(shape, w, B, L + 4)
+    ref.prefill(prompt)
+    ref.step(2)
+    want = _state(ref)
+    side = torch.cuda.Stream()
+    for busy in (200_000, 2_000_000, 100_000_000):   # clocks
+        torch.cuda.synchronize()
+        w_dev = dict(w, embed=w["embed"].cuda(), norm=w["norm"].cuda(), lm_head=w["lm_head"].cuda())
+        eng = _engine(shape, w_dev, B, L + 4)
+        torch.cuda.synchronize()
+        torch.cuda._sleep(busy)
+        with torch.cuda.stream(side):
+            eng.prefill(prompt)
+            eng.step(1)
+        side.synchronize()
+        torch.cuda.synchronize()
+        with torch.cuda.stream(side):
+            eng.step(1)
+            got = _state(eng)
+        side.synchronize()
+        assert eng.status() == 0
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
+        eng.close()
+    ref.close()
