@@ -211,9 +211,9 @@ class DecodeEngine:
         Cn = self.prefill_chunk
         stream = torch.cuda.current_stream().cuda_stream
         if self.B == 1 and L > Cn > 1:
-            if self._pos_bound is None:
-                self._pos_bound = int(self._view("seqlens", (1,), torch.int32).item())
-            pos0 = self._pos_bound
+            # the position on the device: the host's bound does not know of a write through a view of
+            # `seqlens` that the caller has kept
+            pos0 = self._pos_bound = int(self._view("seqlens", (1,), torch.int32).item())
             if pos0 + L > self.S_max:
                 raise ValueError(f"prompt of {L} tokens at position {pos0} exceeds the cache ({self.S_max})")
         if self.prefill_tile and L > 1:

@@ -91,3 +91,32 @@ def test_first_prompt_on_a_side_stream(B):
         assert all(torch.equal(a, b) for a, b in zip(got, want))
         eng.close()
     ref.close()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_prompt_starts_where_the_device_says(dtype):
+    """The caller keeps the view of `seqlens` and writes through it after a prompt: the next prompt of a
+    single sequence starts there, and fits or is refused by it."""
+    shape, L = O.TINY, 21
+    w = O.make_model_weights(shape, seed=6, dtype=dtype)
+    first, second = torch.randint(0, shape.vocab, (2, 1, L), generator=torch.Generator().manual_seed(4))
+    ref = _engine(shape, w, 1, L + 4)
+    ref.prefill(second)
+    eng = _engine(shape, w, 1, L + 4)
+    lens = eng.seqlens
+    eng.prefill(first)
+    assert lens.tolist() == [L]
+    with pytest.raises((IndexError, ValueError)):
+        eng.prefill(second)
+    lens.zero_()
+    eng.prefill(second)                 # the whole cache is free again
+    assert lens.tolist() == [L]
+    assert all(torch.equal(a, b) for a, b in zip(_state(eng), _state(ref)))
+    lens.zero_()
+    eng.prefill(second[:, :10])
+    lens.fill_(8)
+    with pytest.raises((IndexError, ValueError)):
+        eng.prefill(first)              # 8 + 21 positions
+    assert lens.tolist() == [8] and eng.status() == 0
+    eng.close()
+    ref.close()
