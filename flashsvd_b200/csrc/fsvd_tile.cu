@@ -1386,22 +1386,36 @@ static cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, siz
   return launch_pdl_cluster(kern, grid, block, smem, 0u, st, std::forward<Args>(args)...);
 }
 
+// A kernel's dynamic shared-memory limit belongs to a device: raised on the current one, once.
+class SmemLimit {
+  std::atomic<unsigned long long> raised{0};   // a bit per device
+ public:
+  template <typename K>
+  cudaError_t raise(K* kern, int bytes) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess || (dev < 64 && (raised.load(std::memory_order_relaxed) >> dev & 1))) return e;
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess && dev < 64) raised.fetch_or(1ull << dev);
+    return e;
+  }
+};
+
+// (takes the error off the thread, so that no later check of the caller's reports it again)
+static int launch_failed(const char* what) {
+  cudaGetLastError();
+  return fail(FSVD_ERR_CUDA, what);
+}
+
 static int launch_group(const GemmPlan* const* plans, int n, cudaStream_t st);
 static int launch_gemm(const GemmPlan& g, cudaStream_t st) {
   const GemmPlan* one[1] = {&g};
   return launch_group(one, 1, st);
 }
 static int launch_group(const GemmPlan* const* plans, int n, cudaStream_t st) {
-  static bool attr_set = false;
-  static std::mutex mu;
-  {
-    std::lock_guard<std::mutex> lock(mu);
-    if (!attr_set) {
-      if (cudaFuncSetAttribute(tile_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, g_smem_optin - 1024) != cudaSuccess)
-        return fail(FSVD_ERR_CUDA, "cudaFuncSetAttribute failed for the tile kernel");
-      attr_set = true;
-    }
-  }
+  static SmemLimit limit;
+  if (limit.raise(tile_gemm_kernel, g_smem_optin - 1024) != cudaSuccess)
+    return launch_failed("cudaFuncSetAttribute failed for the tile kernel");
   GemmGroup grp;
   memset(&grp, 0, sizeof(grp));
   dim3 grid(1, 1, (unsigned)n);
@@ -1416,7 +1430,7 @@ static int launch_group(const GemmPlan* const* plans, int n, cudaStream_t st) {
   }
   // grid.y = K segments = CTAs of a cluster (the problems of a group have the same number)
   if (launch_pdl_cluster(tile_gemm_kernel, grid, dim3(kThreads), smem, grid.y, st, grp) != cudaSuccess)
-    return fail(FSVD_ERR_CUDA, "tile kernel launch failed");
+    return launch_failed("tile kernel launch failed");
   fsvd_tile_count_launch();
   return 0;
 }
@@ -1580,43 +1594,35 @@ static int plan_layer(LayerPlan& lp, const fsvd_dims& D, const fsvd_layer& Lw, c
 }
 
 template <int DH>
-static void launch_prompt_attn(const PaArgs& pa, int nseq, cudaStream_t st) {
+static cudaError_t launch_prompt_attn(const PaArgs& pa, int nseq, cudaStream_t st) {
   constexpr int smem = 4 * kPaKeys * (DH * 2 + 16);
-  static bool attr_set = false;   // per instantiation; set under the planner's lock or at first use
-  if (!attr_set) {
-    cudaFuncSetAttribute(prompt_attn_kernel<DH>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    attr_set = true;
-  }
+  static SmemLimit limit;
+  const cudaError_t e = limit.raise(prompt_attn_kernel<DH>, smem);
+  if (e != cudaSuccess) return e;
   const int rpb = kPaSlots / (pa.H / pa.Hk);
-  launch_pdl(prompt_attn_kernel<DH>, dim3((unsigned)((pa.L + rpb - 1) / rpb), (unsigned)pa.Hk, (unsigned)nseq), dim3(kPaWarps * 32),
-             (size_t)smem, st, pa);
+  return launch_pdl(prompt_attn_kernel<DH>, dim3((unsigned)((pa.L + rpb - 1) / rpb), (unsigned)pa.Hk, (unsigned)nseq),
+                    dim3(kPaWarps * 32), (size_t)smem, st, pa);
 }
 // rows of nseq sequences, L consecutive positions each
-static void launch_prompt_attn(const PaArgs& pa, int Dh, int nseq, cudaStream_t st) {
-  if (Dh == 128) launch_prompt_attn<128>(pa, nseq, st);
-  else launch_prompt_attn<64>(pa, nseq, st);
+static int launch_prompt_attn(const PaArgs& pa, int Dh, int nseq, cudaStream_t st) {
+  if ((Dh == 128 ? launch_prompt_attn<128>(pa, nseq, st) : launch_prompt_attn<64>(pa, nseq, st)) != cudaSuccess)
+    return launch_failed("attention kernel launch failed");
   fsvd_tile_count_launch();
+  return 0;
 }
 
 template <int DH, bool FULL>
-static void launch_attn_g(const AttnArgs& at, cudaStream_t st) {
-  const unsigned threads = kAttnThreads;
-  const int G = at.H / at.Hk;
-  const unsigned grid = (unsigned)(at.B * at.Hk * at.nsplit);
-  switch (G) {
-    case 1: launch_pdl(batch_attn_kernel<DH, 1, FULL>, dim3(grid), dim3(threads), 0, st, at); break;
-    case 2: launch_pdl(batch_attn_kernel<DH, 2, FULL>, dim3(grid), dim3(threads), 0, st, at); break;
+static cudaError_t launch_attn_g(const AttnArgs& at, cudaStream_t st) {
+  const dim3 grid((unsigned)(at.B * at.Hk * at.nsplit)), threads(kAttnThreads);
+  switch (at.H / at.Hk) {
+    case 1: return launch_pdl(batch_attn_kernel<DH, 1, FULL>, grid, threads, 0, st, at);
+    case 2: return launch_pdl(batch_attn_kernel<DH, 2, FULL>, grid, threads, 0, st, at);
     default: {
       // 4 or 8 heads per kv head: the heads as rows of a tensor-core tile
-      constexpr size_t smem = (size_t)kAttnWarps * 2 * kGqKeys * (DH * 2 + 16);
-      static std::atomic<unsigned long long> attr_set{0};   // per instantiation: a bit per device
-      int dev = 0;
-      cudaGetDevice(&dev);
-      if (dev > 63 || !(attr_set.load(std::memory_order_relaxed) >> dev & 1)) {
-        cudaFuncSetAttribute(gqa_decode_attn_kernel<DH, FULL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (dev <= 63) attr_set.fetch_or(1ull << dev);
-      }
-      launch_pdl(gqa_decode_attn_kernel<DH, FULL>, dim3(grid), dim3(threads), smem, st, at);
+      constexpr int smem = kAttnWarps * 2 * kGqKeys * (DH * 2 + 16);
+      static SmemLimit limit;
+      const cudaError_t e = limit.raise(gqa_decode_attn_kernel<DH, FULL>, smem);
+      return e != cudaSuccess ? e : launch_pdl(gqa_decode_attn_kernel<DH, FULL>, grid, threads, (size_t)smem, st, at);
     }
   }
 }
@@ -1628,15 +1634,10 @@ static PaArgs prompt_args(const AttnArgs& at) {
   return pa;
 }
 static int launch_attn(const AttnArgs& at, cudaStream_t st, bool full = false) {
-  if (at.shared_cache) {
-    // the rows are consecutive positions of one sequence
-    launch_prompt_attn(prompt_args(at), at.Dh, 1, st);
-    if (cudaGetLastError() != cudaSuccess) return fail(FSVD_ERR_CUDA, "attention kernel launch failed");
-    return 0;
-  }
-  if (at.Dh == 128) full ? launch_attn_g<128, true>(at, st) : launch_attn_g<128, false>(at, st);
-  else full ? launch_attn_g<64, true>(at, st) : launch_attn_g<64, false>(at, st);
-  if (cudaGetLastError() != cudaSuccess) return fail(FSVD_ERR_CUDA, "attention kernel launch failed");
+  if (at.shared_cache) return launch_prompt_attn(prompt_args(at), at.Dh, 1, st);   // the rows are consecutive positions of one sequence
+  const cudaError_t e = at.Dh == 128 ? (full ? launch_attn_g<128, true>(at, st) : launch_attn_g<128, false>(at, st))
+                                     : (full ? launch_attn_g<64, true>(at, st) : launch_attn_g<64, false>(at, st));
+  if (e != cudaSuccess) return launch_failed("attention kernel launch failed");
   fsvd_tile_count_launch();
   return 0;
 }
@@ -1647,7 +1648,7 @@ static int launch_reduce(const ReduceArgs& r, int rows, cudaStream_t st) {
   // wide rows are cut into four column slices (a cluster of four CTAs per row)
   const unsigned C = (r.d >= 2048 && r.d % 32 == 0) ? 4u : 1u;
   if (launch_pdl_cluster(exchange_reduce_rows_kernel, dim3((unsigned)rows, C), dim3(256), 0, C > 1 ? C : 0u, st, r) != cudaSuccess)
-    return fail(FSVD_ERR_CUDA, "exchange kernel launch failed");
+    return launch_failed("exchange kernel launch failed");
   fsvd_tile_count_launch();
   return 0;
 }
@@ -1999,7 +2000,7 @@ int fsvd_tile_model_create(const fsvd_dims* dims, const fsvd_layer* layers, cons
   // kernel is raised to the device limit first, outside the capture)
   if (cudaFuncSetAttribute(tile_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, g_smem_optin - 1024) != cudaSuccess) {
     fsvd_tile_model_destroy(m);
-    return fail(FSVD_ERR_CUDA, "cudaFuncSetAttribute failed for the tile kernel");
+    return launch_failed("cudaFuncSetAttribute failed for the tile kernel");
   }
   cudaStream_t cs = nullptr;
   if (cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking) != cudaSuccess) {
@@ -2108,10 +2109,6 @@ int fsvd_tile_prompt_create(const fsvd_dims* dims, const fsvd_layer* layers, con
   const size_t fixed = al256(sizeof(SyncState)) + al256((size_t)D.B * D.d * 2);
   cudaError_t ce = cudaMalloc(&p->fixed, fixed);
   if (ce == cudaSuccess) ce = clear_now(p->fixed, fixed);
-  if (ce == cudaSuccess)
-    ce = cudaFuncSetAttribute(tile_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, g_smem_optin - 1024);
-  if (ce == cudaSuccess)
-    ce = cudaFuncSetAttribute(prompt_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, g_smem_optin - 2048);
   int e = ce == cudaSuccess ? 0 : fail(FSVD_ERR_CUDA, "allocating prompt scratch failed");
   const int HD = D.H * D.Dh, KD = D.Hk * D.Dh;
   p->wmaps.resize((size_t)D.n_layers * PW_COUNT);
@@ -2236,8 +2233,11 @@ static int launch_prompt_gemm(fsvd_tile_prompt* p, int layer, const PgSpec* sp, 
   a.nstages = (g_smem_optin - 4096) / a.stage_bytes;
   if (a.nstages > kPgMaxStages) a.nstages = kPgMaxStages;
   const int grid = a.total < g_sms ? a.total : g_sms;
+  static SmemLimit limit;
+  if (limit.raise(prompt_gemm_kernel, g_smem_optin - 2048) != cudaSuccess)
+    return launch_failed("cudaFuncSetAttribute failed for the prompt kernel");
   if (launch_pdl(prompt_gemm_kernel, dim3((unsigned)grid), dim3(kPgThreads), (size_t)1024 + (size_t)a.nstages * a.stage_bytes, st, a) != cudaSuccess)
-    return fail(FSVD_ERR_CUDA, "prompt kernel launch failed");
+    return launch_failed("prompt kernel launch failed");
   fsvd_tile_count_launch();
   return 0;
 }
@@ -2250,23 +2250,26 @@ int fsvd_tile_prompt_run(fsvd_tile_prompt* p, const int* prompt, int ld, int L, 
   const int passes = (L + most - 1) / most, len = (L + passes - 1) / passes;
   if (int e = prompt_reserve(p, len * D.B)) return e;
   const int HD = D.H * D.Dh, KD = D.Hk * D.Dh, Rqkv = D.Rq + D.Rk + D.Rv;
+  int e = 0;   // after a launch that failed nothing more is launched: no layer over stale rows, no position moved
+  auto launched = [&](cudaError_t ce) {
+    if (ce != cudaSuccess) e = launch_failed("prompt kernel launch failed");
+    else fsvd_tile_count_launch();
+  };
   auto norm = [&](const __nv_bfloat16* x, const void* w, __nv_bfloat16* out, int rows, int mul, int off) {
-    launch_pdl(rmsnorm_rows_kernel<true>, dim3((unsigned)rows), dim3(256), 0, st, x, reinterpret_cast<const __nv_bfloat16*>(w), out, D.d, D.eps,
-               mul, off);
-    fsvd_tile_count_launch();
+    if (!e)
+      launched(launch_pdl(rmsnorm_rows_kernel<true>, dim3((unsigned)rows), dim3(256), 0, st, x, reinterpret_cast<const __nv_bfloat16*>(w),
+                          out, D.d, D.eps, mul, off));
   };
   for (int off = 0; off < L; off += len) {
     const int n = L - off < len ? L - off : len, rows = n * D.B;
-    launch_pdl(prompt_begin_kernel, dim3((unsigned)rows), dim3(128), 0, st, reinterpret_cast<const __nv_bfloat16*>(p->embed), prompt, ld,
-               off, n, (const int*)p->seqlens, p->rowpos, p->rowseq, p->x, D.d, D.vocab);
-    fsvd_tile_count_launch();
+    launched(launch_pdl(prompt_begin_kernel, dim3((unsigned)rows), dim3(128), 0, st, reinterpret_cast<const __nv_bfloat16*>(p->embed),
+                        prompt, ld, off, n, (const int*)p->seqlens, p->rowpos, p->rowseq, p->x, D.d, D.vocab));
     PaArgs pa;
     pa.q = p->qbuf; pa.rowpos = p->rowpos; pa.rowseq = p->rowseq; pa.out = p->attn;
     pa.L = n; pa.H = D.H; pa.Hk = D.Hk; pa.S_max = D.S_max;
     pa.scale_log2 = 1.4426950408889634f / sqrtf((float)D.Dh);
     for (int l = 0; l < D.n_layers; ++l) {
       const fsvd_layer& w = p->lw[l];
-      int e = 0;
       auto gemm = [&](std::initializer_list<PgSpec> sp) {
         if (!e) e = launch_prompt_gemm(p, l, sp.begin(), (int)sp.size(), rows, st);
       };
@@ -2277,7 +2280,7 @@ int fsvd_tile_prompt_run(fsvd_tile_prompt* p, const int* prompt, int ld, int L, 
             {PW_VU, -1, PX_PV, -1, KD, D.Rv, TE_VCACHE, nullptr, nullptr, w.v_cache}});
       pa.kcache = reinterpret_cast<const __nv_bfloat16*>(w.k_cache);
       pa.vcache = reinterpret_cast<const __nv_bfloat16*>(w.v_cache);
-      if (!e) launch_prompt_attn(pa, D.Dh, D.B, st);
+      if (!e) e = launch_prompt_attn(pa, D.Dh, D.B, st);
       gemm({{PW_OV, -1, PX_ATTN, -1, D.Ro, HD, TE_STORE, p->pbuf, nullptr, nullptr}});
       gemm({{PW_OU, -1, PX_PO, -1, D.d, D.Ro, TE_RESID, p->mid, p->x, nullptr}});
       norm(p->mid, w.ln2_w, p->xn, rows, 1, 0);
@@ -2288,20 +2291,19 @@ int fsvd_tile_prompt_run(fsvd_tile_prompt* p, const int* prompt, int ld, int L, 
       if (e) return e;
     }
     if (off + n < L) {
-      launch_pdl(advance_kernel, dim3(1), dim3(128), 0, st, p->seqlens, D.B, n);
-      fsvd_tile_count_launch();
+      launched(launch_pdl(advance_kernel, dim3(1), dim3(128), 0, st, p->seqlens, D.B, n));
+      if (e) return e;
       continue;
     }
     // the last position of every sequence: final norm, head, argmax
     norm(p->x, p->final_norm, prompt_last(p), D.B, n, n - 1);
-    if (int e = launch_gemm(p->head, st)) return e;
-    launch_pdl(argmax_rows_kernel, dim3(D.B), dim3(256), 0, st, (const float*)p->logits, D.vocab, p->tokens, p->token_log,
-               p->step_counter, p->seqlens, p->max_steps, D.B, n);
-    launch_pdl(bump_step_kernel, dim3(1), dim3(1), 0, st, p->step_counter);
-    fsvd_tile_count_launches(2);
+    if (!e) e = launch_gemm(p->head, st);
+    if (!e)
+      launched(launch_pdl(argmax_rows_kernel, dim3(D.B), dim3(256), 0, st, (const float*)p->logits, D.vocab, p->tokens, p->token_log,
+                          p->step_counter, p->seqlens, p->max_steps, D.B, n));
+    if (!e) launched(launch_pdl(bump_step_kernel, dim3(1), dim3(1), 0, st, p->step_counter));
   }
-  if (cudaGetLastError() != cudaSuccess) return fail(FSVD_ERR_CUDA, "kernel launch failed");
-  return 0;
+  return e;
 }
 void* fsvd_tile_prompt_ws(fsvd_tile_prompt* p) { return p->fixed; }
 

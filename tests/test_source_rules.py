@@ -44,3 +44,26 @@ def test_every_device_polling_loop_has_a_budget():
                 window = "\n".join(lines[max(0, i - 6): i + 14])
                 assert "clock64()" in window or "wait_budget" in window or "wait_limit" in window, \
                     f"unbounded polling loop at {path.relative_to(ROOT)}:{i + 1}"
+
+
+def test_shared_memory_limits_are_raised_per_device():
+    """cudaFuncSetAttribute acts on the current device: a flag that says "done" for the process leaves the
+    second GPU of a process without its limit."""
+    for path, text in _texts():
+        if path.suffix not in (".cu", ".cuh", ".h"):
+            continue
+        lines = text.splitlines()
+        for i, line in enumerate(lines):
+            if "cudaFuncSetAttribute(" in line:
+                assert not any(re.search(r"static\s+(std::atomic<bool>|bool)", w) for w in lines[max(0, i - 12): i]), \
+                    f"{path.relative_to(ROOT)}:{i + 1}"
+
+
+def test_a_failed_launch_ends_a_prompt_pass():
+    """No launch of fsvd_tile_prompt_run drops its status: the launches after a failed one would run on stale
+    rows and move the positions."""
+    text = (ROOT / "flashsvd_b200/csrc/fsvd_tile.cu").read_text()
+    body = text[text.index("int fsvd_tile_prompt_run("):]
+    body = body[:body.index("\n}\n")]
+    assert body.count("launch_") >= 8
+    assert not re.findall(r"(?m)^\s*(?:if \(!e\) )?launch_\w+\(", body)
