@@ -320,9 +320,16 @@ __global__ void __launch_bounds__(kPgThreads, 1) prompt_gemm_kernel(const __grid
 // cp.async one block ahead and serve all of them.  S = Q K^T and O += P V on mma.sync m16n8k16 (bf16,
 // fp32 accumulation) with fragments taken by ldmatrix; running softmax in base 2; only blocks that reach
 // past a query's own position are masked.  Query blocks with the longest range start first.
+// The softmax weights of the rows from full_from on meet the value rows with all their 24 bits, as three bf16
+// numbers; those of the rows before are rounded to bf16.  Full are the prompts of several sequences, short
+// blocks of rows and the last kFullRows positions of one sequence (they decide the first token): where a
+// feed token by token or in a few rows has fp32 weights.  The attention of a long prompt is bound by mma.sync:
+// 2041 positions through 4 layers of 32 heads of 128 take 2.85 ms with no full row, 2.90 like this, 3.12 with
+// every row full; six prompts of 190 (all rows full) 1.53 and 1.56 ms.
 constexpr int kPaWarps = 4;
 constexpr int kPaSlots = 16 * kPaWarps;
 constexpr int kPaKeys = 64;
+constexpr int kFullRows = 16;
 
 struct PaArgs {
   const __nv_bfloat16* q;        // [rows, H, Dh], rotated
@@ -332,23 +339,18 @@ struct PaArgs {
   const int* rowseq;             // [rows] cache row, or null: cache row 0
   __nv_bfloat16* out;            // [rows, H, Dh]
   int L, H, Hk, S_max;           // rows per sequence
+  int full_from;                 // rows of a sequence from here on: 24-bit weights
   float scale_log2;              // softmax scale x log2(e)
 };
 
-template <int DH>
-__global__ void __launch_bounds__(kPaWarps * 32) prompt_attn_kernel(const PaArgs a) {
+// Rows r0 .. rlast of the sequence whose first row is seq0.
+template <int DH, bool FULL>
+__device__ __forceinline__ void prompt_attn_rows(const PaArgs& a, unsigned char* pa_smem, int seq0, int r0, int rlast) {
   constexpr int STRIDE = DH * 2 + 16;                 // bytes of a staged row (padded: no bank conflicts)
   constexpr int KS = DH / 16, NT = kPaKeys / 8, DT = DH / 8, PIECES = DH / 8;
   constexpr int STAGE = 2 * kPaKeys * STRIDE;
-  extern __shared__ __align__(16) unsigned char pa_smem[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-  pdl_launch_dependents();
-  pdl_wait();
-  const int G = a.H / a.Hk;
-  const int rpb = kPaSlots / G;                       // positions per CTA
-  const int hk = blockIdx.y, seq0 = blockIdx.z * a.L;  // first row of the sequence
-  const int r0 = (gridDim.x - 1 - blockIdx.x) * rpb;  // first row of the CTA, inside the sequence
-  const int rlast = min(r0 + rpb, a.L) - 1;
+  const int G = a.H / a.Hk, hk = blockIdx.y;
   const int nmax = min(a.rowpos[seq0 + rlast] + 1, a.S_max);   // keys the CTA's last row sees
   const int nfirst = a.rowpos[seq0 + r0] + 1;                  // ... and its first row
   const int m0 = warp * 16 + g;
@@ -462,16 +464,25 @@ __global__ void __launch_bounds__(kPaWarps * 32) prompt_attn_kernel(const PaArgs
     }
 #pragma unroll
     for (int kk = 0; kk < kPaKeys / 16; ++kk) {
-      const uint32_t pa0 = pack_bf16(sc[2 * kk][0], sc[2 * kk][1]), pa1 = pack_bf16(sc[2 * kk][2], sc[2 * kk][3]);
-      const uint32_t pa2 = pack_bf16(sc[2 * kk + 1][0], sc[2 * kk + 1][1]), pa3 = pack_bf16(sc[2 * kk + 1][2], sc[2 * kk + 1][3]);
+      constexpr int W = FULL ? 3 : 1;   // bf16 numbers of a weight
+      uint32_t p[3][4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float x = sc[2 * kk + (i >> 1)][2 * (i & 1)], y = sc[2 * kk + (i >> 1)][2 * (i & 1) + 1];
+        if (FULL) split_bf16(x, y, p[0][i], p[1][i], p[2][i]);
+        else p[0][i] = pack_bf16(x, y);
+      }
       const uint32_t vaddr = vs_s + (uint32_t)((kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * STRIDE + ((lane >> 4) & 1) * 16);
 #pragma unroll
       for (int j = 0; j < DT / 2; ++j) {
         uint32_t b0, b1, b2, b3;
         asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
                      : "=r"(b0), "=r"(b1), "=r"(b2), "=r"(b3) : "r"(vaddr + j * 32));
-        mma_bf16_16816(o[2 * j], pa0, pa1, pa2, pa3, b0, b1);
-        mma_bf16_16816(o[2 * j + 1], pa0, pa1, pa2, pa3, b2, b3);
+#pragma unroll
+        for (int w = W - 1; w >= 0; --w) {
+          mma_bf16_16816(o[2 * j], p[w][0], p[w][1], p[w][2], p[w][3], b0, b1);
+          mma_bf16_16816(o[2 * j + 1], p[w][0], p[w][1], p[w][2], p[w][3], b2, b3);
+        }
       }
     }
     __syncthreads();   // the stage is overwritten by the block after the next
@@ -486,6 +497,18 @@ __global__ void __launch_bounds__(kPaWarps * 32) prompt_attn_kernel(const PaArgs
 #pragma unroll
     for (int d = 0; d < DT; ++d) *reinterpret_cast<uint32_t*>(op + d * 8) = pack_bf16(o[d][2 * i] * inv, o[d][2 * i + 1] * inv);
   }
+}
+
+template <int DH>
+__global__ void __launch_bounds__(kPaWarps * 32, DH == 64 ? 4 : 3) prompt_attn_kernel(const PaArgs a) {
+  extern __shared__ __align__(16) unsigned char pa_smem[];
+  pdl_launch_dependents();
+  pdl_wait();
+  const int rpb = kPaSlots / (a.H / a.Hk);            // positions per CTA
+  const int r0 = (gridDim.x - 1 - blockIdx.x) * rpb;  // first row of the CTA, inside the sequence
+  const int rlast = min(r0 + rpb, a.L) - 1;
+  if (rlast >= a.full_from) prompt_attn_rows<DH, true>(a, pa_smem, blockIdx.z * a.L, r0, rlast);
+  else prompt_attn_rows<DH, false>(a, pa_smem, blockIdx.z * a.L, r0, rlast);
 }
 
 }  // namespace fsvd_tile

@@ -121,7 +121,22 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<const uint32_t*>(&v);
 }
-
+// Two fp32 numbers as sums of three bf16 numbers each (packed like pack_bf16): hi and mid cut off 8 significant
+// bits, lo is what is left of the 24, so that nothing is lost (numbers below 2^-110 aside).  Products with
+// bf16 numbers are exact in an MMA: its result is that of the fp32 weights.
+__device__ __forceinline__ void split_bf16(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+  const uint32_t cut = 0xffff0000u;
+  uint32_t a = __float_as_uint(x), b = __float_as_uint(y);
+  hi = __byte_perm(a, b, 0x7632);
+  x -= __uint_as_float(a & cut);
+  y -= __uint_as_float(b & cut);
+  a = __float_as_uint(x);
+  b = __float_as_uint(y);
+  mid = __byte_perm(a, b, 0x7632);
+  x -= __uint_as_float(a & cut);
+  y -= __uint_as_float(b & cut);
+  lo = __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632);
+}
 
 // Bounded mbarrier wait; false when the budget ran out or the CTA has given up already.
 __device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, volatile int* giveup, int* status, long long limit, int code) {

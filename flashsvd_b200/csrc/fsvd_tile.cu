@@ -1604,7 +1604,8 @@ static cudaError_t launch_prompt_attn(const PaArgs& pa, int nseq, cudaStream_t s
                     dim3(kPaWarps * 32), (size_t)smem, st, pa);
 }
 // rows of nseq sequences, L consecutive positions each
-static int launch_prompt_attn(const PaArgs& pa, int Dh, int nseq, cudaStream_t st) {
+static int launch_prompt_attn(PaArgs pa, int Dh, int nseq, cudaStream_t st) {
+  pa.full_from = nseq > 1 ? 0 : pa.L - kFullRows;
   if ((Dh == 128 ? launch_prompt_attn<128>(pa, nseq, st) : launch_prompt_attn<64>(pa, nseq, st)) != cudaSuccess)
     return launch_failed("attention kernel launch failed");
   fsvd_tile_count_launch();
