@@ -1,8 +1,8 @@
 """`flash_decode` on its own against softmax attention in 64 bits.
 
-Tolerance: the output is one bf16 rounding (8 significant bits: 2^-8 of the value) of sums whose weights are kept to 32 bits or
-as two bf16 numbers (2^-16), so 2^-8 |ref| plus 5e-5 of the largest value; weights rounded to bf16 miss
-it.  A cache that does not start on a 16-byte boundary takes the interpreter's stage and must agree too."""
+Tolerance: the output is one bf16 rounding (8 significant bits: 2^-8 of the value) of sums whose weights are kept to 32 bits,
+so 2^-8 |ref| plus 5e-5 of the largest value; weights rounded to bf16 miss it (test_gpu_softmax_weights.py
+tells 24 bits from 16).  A cache that does not start on a 16-byte boundary takes the interpreter's stage and must agree too."""
 import pytest
 import torch
 

@@ -74,3 +74,23 @@ def test_prompt_rows(H, Hk, Dh, B):
     got = out.double().cpu()[-16:].view(-1, H, Dh)
     n = Dh - 1                               # (the last dimension of the last head holds the residual)
     assert bool(((got - ref).abs() <= tol)[..., :n].all())
+
+
+@pytest.mark.parametrize("n", [3, 70, 1200])
+@pytest.mark.parametrize("H,Hk,Dh", [(4, 4, 64), (4, 2, 64), (4, 1, 64), (8, 2, 128), (8, 1, 128)])
+def test_flash_decode(H, Hk, Dh, n):
+    """The op, in one split and in several: the three keys are the last ones, all others score below -1000."""
+    from flashsvd_b200 import ops
+
+    dev, dtype, qn = torch.device("cuda:0"), torch.bfloat16, 16
+    key, values, ref, tol = _case(qn, Dh, H + n)
+    q = torch.zeros(1, H, Dh, dtype=dtype, device=dev)
+    q[..., 0] = qn
+    k, v = (torch.zeros(1, n, Hk, Dh, dtype=dtype, device=dev) for _ in range(2))
+    k[:, :-3, :, 0] = -64.0 * qn
+    k[:, -3, :, 0] = key
+    v[:, :-3] = 1.0
+    v[0, -3:] = values.to(dev)[:, None]
+    ws = ops.make_workspace(ops.make_dims(dtype=dtype, B=1, H=H, Hk=Hk, Dh=Dh, S_max=n), dev)
+    out = ops.flash_decode(q, k, v, torch.tensor([n], dtype=torch.int32, device=dev), ws)
+    assert bool(((out[0].double().cpu() - ref).abs() <= tol).all())
