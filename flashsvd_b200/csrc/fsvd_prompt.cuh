@@ -487,16 +487,31 @@ __device__ __forceinline__ void prompt_attn_rows(const PaArgs& a, unsigned char*
     }
     __syncthreads();   // the stage is overwritten by the block after the next
   }
+  unsigned again[2];   // rows (four lanes each) that met the infinite value of a position they do not see, or of one with a short weight
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
     lrow[i] += __shfl_xor_sync(0xffffffffu, lrow[i], 1);
     lrow[i] += __shfl_xor_sync(0xffffffffu, lrow[i], 2);
-    if (nl[i] == 0) continue;
+    bool none = false;   // "no number" among this thread's sums
+#pragma unroll
+    for (int d = 0; d < DT; ++d) none |= o[d][2 * i] != o[d][2 * i] || o[d][2 * i + 1] != o[d][2 * i + 1];
+    again[i] = __ballot_sync(0xffffffffu, nl[i] > 0 && none);
+    if (nl[i] == 0 || (again[i] >> (lane & 28) & 15u)) continue;
     const float inv = lrow[i] > 0.0f ? 1.0f / lrow[i] : 0.0f;
     __nv_bfloat16* op = a.out + ((size_t)rowq[i] * a.H + headq[i]) * DH + 2 * t;
 #pragma unroll
     for (int d = 0; d < DT; ++d) *reinterpret_cast<uint32_t*>(op + d * 8) = pack_bf16(o[d][2 * i] * inv, o[d][2 * i + 1] * inv);
   }
+#pragma unroll 1
+  for (int m = 0; m < 16 && (again[0] | again[1]); ++m)   // rows 0 .. 7 and 8 .. 15 of the warp
+    if ((m < 8 ? again[0] : again[1]) >> (4 * (m & 7)) & 15u) {
+      const int r = r0 + (warp * 16 + m) / G, n = min(nfirst + r - r0, a.S_max);
+      const size_t at = ((size_t)(seq0 + r) * a.H + hk * G + (warp * 16 + m) % G) * DH;
+      float acc[DH / 32], mm, ll;
+      attn_one_row<DH>(a.q + at, kbase, vbase, rowstride, 0, n, n, n, a.scale_log2 * 0.6931471805599453f, acc, &mm, &ll);
+#pragma unroll
+      for (int e = 0; e < DH / 32; ++e) a.out[at + lane * (DH / 32) + e] = __float2bfloat16_rn(acc[e] / ll);
+    }
 }
 
 template <int DH>

@@ -703,6 +703,42 @@ __device__ __forceinline__ void ld_row<2>(const __nv_bfloat16* row, int lane, fl
   f[0] = __uint_as_float(w << 16); f[1] = __uint_as_float(w & 0xffff0000u);
 }
 
+// One query vector over the keys [k0, k0 + block) below `end`, k0 = begin, begin + stride, ..., by one warp in plain
+// fp32; lane t gets dims DPL t .. DPL t + DPL - 1 of the sum over the values, the running maximum and the running sum.
+// The tensor cores multiply every value row of a tile by every weight of it, the zeros of masked positions and of a
+// weight's lower parts too, and 0 times an infinity is no number: the kernels take a row that came out as one
+// again through here, where a position that a query does not see takes no part.  (Finite rows never do.)
+template <int DH>
+__device__ __noinline__ void attn_one_row(const __nv_bfloat16* q, const __nv_bfloat16* kbase, const __nv_bfloat16* vbase, size_t rowstride,
+                                          int begin, int end, int block, int stride, float scale, float* acc, float* m, float* l) {
+  constexpr int DPL = DH / 32;
+  const int lane = threadIdx.x & 31;
+  float qf[DPL], o[DPL], mm = -INFINITY, ll = 0.0f;
+  ld_row<DPL>(q, lane, qf);
+#pragma unroll
+  for (int e = 0; e < DPL; ++e) o[e] = 0.0f;
+  for (int k0 = begin; k0 < end; k0 += stride)
+    for (int k = k0; k < min(k0 + block, end); ++k) {
+      float kf[DPL], vf[DPL], s = 0.0f;
+      ld_row<DPL>(kbase + (size_t)k * rowstride, lane, kf);
+      ld_row<DPL>(vbase + (size_t)k * rowstride, lane, vf);
+#pragma unroll
+      for (int e = 0; e < DPL; ++e) s += qf[e] * kf[e];
+#pragma unroll
+      for (int x = 16; x > 0; x >>= 1) s += __shfl_xor_sync(0xffffffffu, s, x);
+      s *= scale;
+      const float mn = fmaxf(mm, s), corr = expf(mm - mn), p = expf(s - mn);
+      mm = mn;
+      ll = ll * corr + p;
+#pragma unroll
+      for (int e = 0; e < DPL; ++e) o[e] = o[e] * corr + p * vf[e];
+    }
+#pragma unroll
+  for (int e = 0; e < DPL; ++e) acc[e] = o[e];
+  *m = mm;
+  *l = ll;
+}
+
 template <int DH, int G, bool FULL>
 __global__ void __launch_bounds__(kAttnThreads) batch_attn_kernel(const AttnArgs a) {
   constexpr int DPL = DH / 32;
@@ -742,9 +778,15 @@ __global__ void __launch_bounds__(kAttnThreads) batch_attn_kernel(const AttnArgs
     float kf[kKeyGroup][DPL], vf[kKeyGroup][DPL];
 #pragma unroll
     for (int i = 0; i < kKeyGroup; ++i) {
-      const int row = c0 + (i < cn ? i : cn - 1);   // past the end: the last row again, weighted 0 below
+      const int row = c0 + (i < cn ? i : cn - 1);   // past the end: the last row again, masked below
       ld_row<DPL>(kbase + (size_t)row * rowstride, lane, kf[i]);
       ld_row<DPL>(vbase + (size_t)row * rowstride, lane, vf[i]);
+    }
+    if (cn < kKeyGroup) {   // (the loads above stay unconditional: with a branch each the kernel took twice the time)
+#pragma unroll
+      for (int i = 0; i < kKeyGroup; ++i)
+#pragma unroll
+        for (int e = 0; e < DPL; ++e) vf[i][e] = i < cn ? vf[i][e] : 0.0f;   // its weight is 0, and 0 times an infinity is no number
     }
 #pragma unroll
     for (int g = 0; g < G; ++g) {
@@ -1009,6 +1051,25 @@ __global__ void __launch_bounds__(kAttnThreads, 3) gqa_decode_attn_kernel(const 
       mine[DH] = mrow;
       mine[DH + 1] = lrow;
     }
+  }
+  if (FULL) {
+    bool none = false;   // "no number" among this thread's sums
+#pragma unroll
+    for (int d = 0; d < DT; ++d) none |= o[d][0] != o[d][0] || o[d][1] != o[d][1];
+    unsigned again = __ballot_sync(0xffffffffu, g < G && none);
+    for (int gg = 0; again; ++gg, again >>= 4)
+      if (again & 15u) {
+        float acc[DH / 32], mm, ll;
+        attn_one_row<DH>(a.q + ((size_t)b * a.H + hk * G + gg) * DH, kbase, vbase, rowstride, j0 + warp * kGqKeys, j1, kGqKeys,
+                         kAttnWarps * kGqKeys, a.scale, acc, &mm, &ll);
+        float* mine = wpart + ((size_t)warp * G + gg) * rec;
+#pragma unroll
+        for (int e = 0; e < DH / 32; ++e) mine[lane * (DH / 32) + e] = acc[e];
+        if (lane == 0) {
+          mine[DH] = mm;
+          mine[DH + 1] = ll;
+        }
+      }
   }
   __syncthreads();
   const int nsplit = a.nsplit;

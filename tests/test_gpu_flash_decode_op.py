@@ -53,3 +53,23 @@ def test_flash_decode_keeps_the_weights_in_32_bits(B, H, Hk, Dh, S, lens, offset
         assert bool(((out.double().cpu() - ref).abs() <= bound).all())
     again = ops.flash_decode(q.to(dev), place(k), place(v), (n - 1).to(dev), ws, seqlen_add=1)
     assert torch.equal(again, out)
+
+
+@pytest.mark.parametrize("H,Hk,Dh", [(4, 4, 64), (4, 2, 128), (4, 1, 64), (8, 1, 128)])
+@pytest.mark.parametrize("n", [1, 9, 33, 61, 700])
+def test_infinity_in_the_last_value_row(H, Hk, Dh, n):
+    """An infinity among the values of the last visible position gives an infinity in that dimension (its weight
+    is positive), and nothing else: rows past the end of a split take no part."""
+    from flashsvd_b200 import ops
+
+    dev = torch.device("cuda:0")
+    gen = torch.Generator().manual_seed(n)
+    q = torch.randn(1, H, Dh, generator=gen).to(torch.bfloat16)
+    k, v = (torch.randn(1, n, Hk, Dh, generator=gen).to(torch.bfloat16) for _ in range(2))
+    v[0, -1, :, 5], v[0, -1, :, Dh - 1] = float("inf"), float("-inf")
+    ref = _reference(q, k, v, [n], Dh ** -0.5)
+    ws = ops.make_workspace(ops.make_dims(dtype=torch.bfloat16, B=1, H=H, Hk=Hk, Dh=Dh, S_max=n), dev)
+    out = ops.flash_decode(q.to(dev), k.to(dev), v.to(dev), torch.tensor([n], dtype=torch.int32, device=dev), ws).double().cpu()
+    assert bool((out[..., 5] == float("inf")).all()) and bool((out[..., Dh - 1] == float("-inf")).all())
+    rest = [i for i in range(Dh) if i not in (5, Dh - 1)]
+    assert bool(((out - ref).abs() <= ref.abs() * 2.0 ** -8 + 5e-5 * 5.0)[..., rest].all())
