@@ -1247,6 +1247,7 @@ int fsvd_model_create(const fsvd_dims* dims, const fsvd_layer* layers, const voi
     s.flags = SF_OUT_T;
     s.tokens = m->tokens;
     s.vocab = D.vocab;
+    s.best = argmax_keys(m->ws, m->L);
     b.push(s);
   }
   for (int l = 0; l < D.n_layers; ++l) {
@@ -1413,7 +1414,7 @@ int fsvd_model_reset_sync(fsvd_model* m, void* stream) {
   if (!m) return fail(FSVD_ERR_ARG, "null model");
   if (m->prompt) return fsvd_workspace_clear_status(fsvd_tile_prompt_ws(m->prompt), stream);
   if (m->tile) return fsvd_tile_model_reset(m->tile, stream);
-  CUDA_TRY(cudaMemsetAsync(m->ws + m->L.sync, 0, al256(sizeof(SyncState)), (cudaStream_t)stream));   // (and the argmax keys)
+  CUDA_TRY(cudaMemsetAsync(m->ws + m->L.sync, 0, sizeof(SyncState), (cudaStream_t)stream));
   CUDA_TRY(cudaMemsetAsync(m->ws + m->L.counters, 0, kCounterBytes, (cudaStream_t)stream));
   return 0;
 }

@@ -1403,6 +1403,9 @@ template <typename T>
 __device__ __forceinline__ void run_embed(const Stage& st, int gtid, int gthreads) {
   using X = TT<T>;
   const int d = st.P, B = st.B;
+  // The keys of the step's argmax start at 0 here and not where the last step left them: in a step whose waits ran
+  // out, a CTA may have added to them after they were read.
+  if (st.best && gtid < B) st.best[gtid] = 0ull;
   for (int i = gtid; i < B * d; i += gthreads) {
     const int b = i / d, k = i - b * d;
     int tok = st.tokens[b];
@@ -1420,7 +1423,6 @@ static __device__ __forceinline__ void run_argmax(const Stage& st, int tid) {
   __syncwarp();
   if (tid < st.B) {
     const unsigned long long key = __ldcg(st.best + tid);
-    st.best[tid] = 0ull;
     const int bi = key ? (int)~(uint32_t)key : 0;
     st.tokens[tid] = bi;
     if (st.token_log && step < st.max_steps) st.token_log[(size_t)step * st.B + tid] = bi;

@@ -102,7 +102,7 @@ struct alignas(16) Stage {
   int* step_counter;     // incremented once per ST_ARGMAX
   int* seqlens_rw;       // [B] incremented by ST_ARGMAX
   int vocab, max_steps;
-  unsigned long long* best;   // [B] running argmax keys: written by the lm_head stage (else null), read and zeroed by ST_ARGMAX
+  unsigned long long* best;   // [B] running argmax keys of a model step: zeroed by ST_EMBED, raised by the lm_head stage, read by ST_ARGMAX; else null
 };
 static_assert(sizeof(Stage) == 288, "Stage has no implicit padding");
 

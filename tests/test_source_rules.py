@@ -67,3 +67,16 @@ def test_a_failed_launch_ends_a_prompt_pass():
     body = body[:body.index("\n}\n")]
     assert body.count("launch_") >= 8
     assert not re.findall(r"(?m)^\s*(?:if \(!e\) )?launch_\w+\(", body)
+
+
+def test_argmax_keys_start_every_step_at_zero():
+    """A step whose waits ran out leaves the argmax keys of its last CTAs behind; launches after it work
+    normally, so no step may begin with the keys of the one before."""
+    kernel = (ROOT / "flashsvd_b200/csrc/fsvd_kernel.cuh").read_text()
+    embed = kernel[kernel.index("void run_embed("):]
+    embed = embed[:embed.index("\n}\n")]
+    assert "st.best[gtid] = 0ull" in embed
+    api = (ROOT / "flashsvd_b200/csrc/fsvd_api.cu").read_text()
+    for stage in ("ST_EMBED", "ST_ARGMAX"):
+        block = api[api.index(f"s.type = {stage};"):]
+        assert "s.best = argmax_keys(" in block[:block.index("b.push(s);")], stage
