@@ -2117,9 +2117,10 @@ int fsvd_tile_model_reset(fsvd_tile_model* m, void* stream) {
 }
 
 // ---- prompt pass (kernels in fsvd_prompt.cuh)
-// Rows of a pass at most; what a pass keeps per row is allocated for as many rows as the longest prompt so
-// far needed.
+// Rows of a pass at most.  What a pass keeps per row is allocated with the program, for the longest pass its
+// caches can take: a run allocates and frees nothing, and a graph that has captured one keeps valid addresses.
 constexpr int kPromptRows = 2048;
+static int prompt_pass_positions(const fsvd_dims& D) { return std::min(D.S_max, std::max(1, kPromptRows / D.B)); }
 enum PromptW { PW_QKV, PW_QU, PW_KU, PW_VU, PW_OV, PW_OU, PW_UG, PW_GU, PW_UU, PW_DV, PW_DU, PW_COUNT };
 enum PromptX { PX_XN, PX_PQ, PX_PK, PX_PV, PX_ATTN, PX_PO, PX_PUP, PX_PGATE, PX_HACT, PX_PD, PX_COUNT };
 
@@ -2132,10 +2133,10 @@ struct fsvd_tile_prompt {
   // the decode model's buffers: positions are read and advanced, the last position's token and logits go there
   int *tokens = nullptr, *seqlens = nullptr, *step_counter = nullptr, *token_log = nullptr;
   float* logits = nullptr;
-  int max_steps = 0, cap = 0;
+  int max_steps = 0;
   long long wait_limit = 0;
   char* fixed = nullptr;             // status words, normalised last rows
-  char* ws = nullptr;                // [cap] rows of everything below
+  char* ws = nullptr;                // rows of everything below
   int *rowpos = nullptr, *rowseq = nullptr;
   __nv_bfloat16 *x = nullptr, *mid = nullptr, *xn = nullptr, *pbuf = nullptr, *qbuf = nullptr, *attn = nullptr, *hact = nullptr;
   GemmPlan head;
@@ -2149,6 +2150,35 @@ int fsvd_tile_prompt_destroy(fsvd_tile_prompt* p) {
   cudaFree(p->fixed);
   cudaFree(p->ws);
   delete p;
+  return 0;
+}
+
+// Scratch for the rows of the longest pass.
+static int prompt_scratch(fsvd_tile_prompt* p) {
+  const fsvd_dims& D = p->D;
+  // whole tiles: with 2045 rows, the last tile partly outside the tensor maps, 2041 positions through 4 layers of the 7B
+  // shape took 3.07 ms, with 2048 rows 2.92
+  const int rows = (prompt_pass_positions(D) * D.B + kTileM - 1) / kTileM * kTileM;
+  const int HD = D.H * D.Dh, Rqkv = D.Rq + D.Rk + D.Rv, Rmlp = D.Ru + D.Rg;
+  const int pw = imax(imax(Rqkv, Rmlp), imax(D.Ro, D.Rd));
+  const size_t n = (size_t)rows;
+  const size_t bytes[] = {n * 4, n * 4, n * D.d * 2, n * D.d * 2, n * D.d * 2, n * pw * 2, n * HD * 2, n * HD * 2, n * D.I * 2};
+  size_t total = 0, off[9];
+  for (int i = 0; i < 9; ++i) {
+    off[i] = total;
+    total += al256(bytes[i]);
+  }
+  // (not cleared: the rows past a pass's last one, multiplied too, reach only accumulator rows that are never stored)
+  if (cudaMalloc(&p->ws, total) != cudaSuccess) return launch_failed("allocating prompt scratch failed");
+  p->rowpos = reinterpret_cast<int*>(p->ws + off[0]);
+  p->rowseq = reinterpret_cast<int*>(p->ws + off[1]);
+  __nv_bfloat16** t[] = {&p->x, &p->mid, &p->xn, &p->pbuf, &p->qbuf, &p->attn, &p->hact};
+  for (int i = 0; i < 7; ++i) *t[i] = reinterpret_cast<__nv_bfloat16*>(p->ws + off[2 + i]);
+  const struct { const __nv_bfloat16* base; int K, ld; } f[PX_COUNT] = {
+      {p->xn, D.d, D.d}, {p->pbuf, D.Rq, Rqkv}, {p->pbuf + D.Rq, D.Rk, Rqkv}, {p->pbuf + D.Rq + D.Rk, D.Rv, Rqkv}, {p->attn, HD, HD},
+      {p->pbuf, D.Ro, D.Ro}, {p->pbuf, D.Ru, Rmlp}, {p->pbuf + D.Ru, D.Rg, Rmlp}, {p->hact, D.I, D.I}, {p->pbuf, D.Rd, D.Rd}};
+  for (int i = 0; i < PX_COUNT; ++i)
+    if (int e = encode_sw128(&p->xmaps[i], f[i].base, rows, f[i].K, f[i].ld, kTileM)) return e;
   return 0;
 }
 
@@ -2173,7 +2203,7 @@ int fsvd_tile_prompt_create(const fsvd_dims* dims, const fsvd_layer* layers, con
   const size_t fixed = al256(sizeof(SyncState)) + al256((size_t)D.B * D.d * 2);
   cudaError_t ce = cudaMalloc(&p->fixed, fixed);
   if (ce == cudaSuccess) ce = clear_now(p->fixed, fixed);
-  int e = ce == cudaSuccess ? 0 : fail(FSVD_ERR_CUDA, "allocating prompt scratch failed");
+  int e = ce == cudaSuccess ? prompt_scratch(p) : launch_failed("allocating prompt scratch failed");
   const int HD = D.H * D.Dh, KD = D.Hk * D.Dh;
   p->wmaps.resize((size_t)D.n_layers * PW_COUNT);
   for (int l = 0; l < D.n_layers && !e; ++l) {
@@ -2194,42 +2224,6 @@ int fsvd_tile_prompt_create(const fsvd_dims* dims, const fsvd_layer* layers, con
     return e;
   }
   *out = p;
-  return 0;
-}
-
-// Scratch for `rows` rows of a pass.
-static int prompt_reserve(fsvd_tile_prompt* p, int rows) {
-  if (rows <= p->cap) return 0;
-  int cap = 256;
-  while (cap < rows) cap *= 2;
-  const fsvd_dims& D = p->D;
-  const int HD = D.H * D.Dh, Rqkv = D.Rq + D.Rk + D.Rv, Rmlp = D.Ru + D.Rg;
-  const int pw = imax(imax(Rqkv, Rmlp), imax(D.Ro, D.Rd));
-  const size_t n = (size_t)cap;
-  const size_t bytes[] = {n * 4, n * 4, n * D.d * 2, n * D.d * 2, n * D.d * 2, n * pw * 2, n * HD * 2, n * HD * 2, n * D.I * 2};
-  size_t total = 0, off[9];
-  for (int i = 0; i < 9; ++i) {
-    off[i] = total;
-    total += al256(bytes[i]);
-  }
-  char* ws = nullptr;
-  if (cudaMalloc(&ws, total) != cudaSuccess) return fail(FSVD_ERR_CUDA, "allocating prompt scratch failed");
-  // (not cleared: the rows past a pass's last one, multiplied too, reach only accumulator rows that are never stored)
-  cudaFree(p->ws);   // (waits for the passes that still use it)
-  p->ws = ws;
-  p->cap = cap;
-  p->rowpos = reinterpret_cast<int*>(ws + off[0]);
-  p->rowseq = reinterpret_cast<int*>(ws + off[1]);
-  __nv_bfloat16** t[] = {&p->x, &p->mid, &p->xn, &p->pbuf, &p->qbuf, &p->attn, &p->hact};
-  for (int i = 0; i < 7; ++i) *t[i] = reinterpret_cast<__nv_bfloat16*>(ws + off[2 + i]);
-  const struct { const __nv_bfloat16* base; int K, ld; } f[PX_COUNT] = {
-      {p->xn, D.d, D.d}, {p->pbuf, D.Rq, Rqkv}, {p->pbuf + D.Rq, D.Rk, Rqkv}, {p->pbuf + D.Rq + D.Rk, D.Rv, Rqkv}, {p->attn, HD, HD},
-      {p->pbuf, D.Ro, D.Ro}, {p->pbuf, D.Ru, Rmlp}, {p->pbuf + D.Ru, D.Rg, Rmlp}, {p->hact, D.I, D.I}, {p->pbuf, D.Rd, D.Rd}};
-  for (int i = 0; i < PX_COUNT; ++i)
-    if (int e = encode_sw128(&p->xmaps[i], f[i].base, cap, f[i].K, f[i].ld, kTileM)) {
-      p->cap = 0;
-      return e;
-    }
   return 0;
 }
 
@@ -2310,9 +2304,8 @@ static int launch_prompt_gemm(fsvd_tile_prompt* p, int layer, const PgSpec* sp, 
 int fsvd_tile_prompt_run(fsvd_tile_prompt* p, const int* prompt, int ld, int L, void* stream) {
   const fsvd_dims& D = p->D;
   cudaStream_t st = (cudaStream_t)stream;
-  const int most = kPromptRows / D.B > 1 ? kPromptRows / D.B : 1;   // positions of a pass
+  const int most = prompt_pass_positions(D);
   const int passes = (L + most - 1) / most, len = (L + passes - 1) / passes;
-  if (int e = prompt_reserve(p, len * D.B)) return e;
   const int HD = D.H * D.Dh, KD = D.Hk * D.Dh, Rqkv = D.Rq + D.Rk + D.Rv;
   int e = 0;   // after a launch that failed nothing more is launched: no layer over stale rows, no position moved
   auto launched = [&](cudaError_t ce) {

@@ -216,7 +216,9 @@ class DecodeEngine:
             pos0 = self._pos_bound = int(self._view("seqlens", (1,), torch.int32).item())
             if pos0 + L > self.S_max:
                 raise ValueError(f"prompt of {L} tokens at position {pos0} exceeds the cache ({self.S_max})")
-        if self.prefill_tile and L > 1:
+        # (its program is made by the first prompt, which allocates: a first prompt inside a graph capture goes
+        # token by token)
+        if self.prefill_tile and L > 1 and (self.prefill_tile in self._chunks or not torch.cuda.is_current_stream_capturing()):
             handle = self._prompt_program()
             self._reserve_positions(L)
             check(self.lib.fsvd_prompt_run(handle, prompt.data_ptr(), L, L, stream))

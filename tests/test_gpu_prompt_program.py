@@ -120,3 +120,51 @@ def test_prompt_starts_where_the_device_says(dtype):
     assert lens.tolist() == [8] and eng.status() == 0
     eng.close()
     ref.close()
+
+
+@pytest.mark.parametrize("B", [2, 12])
+def test_prompts_in_captured_graphs(B):
+    """A prompt captured into a graph replays with the values of a direct call, also after longer prompts have
+    gone through the engine in between; an engine's first prompt can be captured too (token by token:
+    nothing may be allocated there), where one launch per token can."""
+    shape, L = O.TINY_GQA, 40
+    w = O.make_model_weights(shape, seed=8, dtype=torch.bfloat16)
+    long, prompt = torch.randint(0, shape.vocab, (2, B, 3 * L), generator=torch.Generator().manual_seed(B), dtype=torch.int32).cuda()
+    prompt = prompt[:, :L].contiguous()
+    ref = _engine(shape, w, B, 3 * L)
+    ref.prefill(prompt)
+    want = _state(ref)
+    eng = _engine(shape, w, B, 3 * L)
+    lens = eng.seqlens
+    eng.prefill(prompt[:, :5])
+    eng.reset()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        eng.prefill(prompt)
+    eng.reset()
+    eng.prefill(long)
+    for c in (*eng.key_cache, *eng.value_cache):
+        c.zero_()
+    for _ in range(2):
+        lens.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert eng.status() == 0
+        assert all(torch.equal(a, b) for a, b in zip(_state(eng), want))
+    graph.reset()
+    eng.close()
+    if B == 2:
+        first = _engine(shape, w, B, 3 * L)
+        tokenwise = _engine(shape, w, B, 3 * L, prefill_chunk=1)
+        tokenwise.prefill(prompt)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            first.prefill(prompt)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert first.status() == 0
+        assert all(torch.equal(a, b) for a, b in zip(_state(first), _state(tokenwise)))
+        graph.reset()
+        first.close()
+        tokenwise.close()
+    ref.close()
