@@ -11,9 +11,9 @@
 
 namespace {
 
-template <typename T, bool Q4>
-cudaError_t launch_impl(const LaunchArgs& a) {
-  auto kern = fsvd::fsvd_decode_kernel<T, Q4>;
+template <typename T, bool Q4, bool MODEL>
+cudaError_t launch_kernel(const LaunchArgs& a) {
+  auto kern = fsvd::fsvd_decode_kernel<T, Q4, MODEL>;
   // largest dynamic shared-memory size the kernel has been opted into, per device
   static size_t attr_smem[16] = {0};
   static std::mutex attr_mu;
@@ -45,6 +45,10 @@ cudaError_t launch_impl(const LaunchArgs& a) {
                             a.small_maps ? *a.small_maps : empty_maps, a.small ? 1 : 0, a.nstages,
                             a.sync, a.xstride, a.part_bytes, a.vec_bytes, a.nslots, a.slot_bytes, a.trace,
                             a.wait_limit);
+}
+template <typename T, bool Q4>
+cudaError_t launch_impl(const LaunchArgs& a) {
+  return a.small ? launch_kernel<T, Q4, false>(a) : launch_kernel<T, Q4, true>(a);
 }
 
 }  // namespace

@@ -872,7 +872,7 @@ struct StageCtx {
 };
 
 // One GEMV stage, consumer warps.  Returns the number of boxes of this CTA in the stage.
-template <typename T, bool Q4>
+template <typename T, bool Q4, bool MODEL>
 __device__ __forceinline__ int gemv_stage(const Stage& st, const StageCtx cx) {
   using X = TT<T>;
   constexpr int BOXCOLS = kBoxRowBytes / (int)sizeof(T);
@@ -1079,7 +1079,7 @@ __device__ __forceinline__ int gemv_stage(const Stage& st, const StageCtx cx) {
       for (int k2 = 0; k2 < KK; ++k2) sum1 += src[(size_t)(KK + k2) * rowsB];
     gemv_epilogue<T>(st, p, b, seg, sum0, sum1, ax);
   }
-  if (st.best) best_logits<T>(st, cx.part, bp.nu, bp.first, KK, tid);
+  if (MODEL && st.best) best_logits<T>(st, cx.part, bp.nu, bp.first, KK, tid);
   trace_mark(cx.trow, 11);
   return bp.nbox;
 }
@@ -1444,7 +1444,11 @@ static __device__ __forceinline__ void run_argmax(const Stage& st, int tid) {
 // Stage timeline (optional): trace[(s*grid + cta)*16 + k] = globaltimer at: 0 stage entry,
 // 1 grid barrier passed, 2 vector staged, 3 stage done, 4 vector words arrived, 5 norm reduced,
 // 7 boxes consumed.
-template <typename T, bool Q4>
+// MODEL: whole-model steps (device-resident programs).  A launch of one op or layer has no embedding, no logits and no
+// argmax, and its kernel does without their code (the interpreter is bound by instruction fetch where its stages are short: the
+// fused MLP of d 1024, I 2816, rank 376 takes 24.95 us with it and 24.64 without in fp32, two rows; that of the 7B shape
+// in bf16 39.36 and 39.21).
+template <typename T, bool Q4, bool MODEL>
 __global__ void __launch_bounds__(kThreads, 1)
 fsvd_decode_kernel(const Stage* __restrict__ prog_global, const __grid_constant__ SmallProgram small,
                    const unsigned char* __restrict__ maps_global, const __grid_constant__ SmallMaps small_maps,
@@ -1552,7 +1556,7 @@ fsvd_decode_kernel(const Stage* __restrict__ prog_global, const __grid_constant_
         cx.giveup = giveup;
         cx.pc = pc;
         cx.trow = trow;
-        seq_base += (unsigned)gemv_stage<T, Q4>(st, cx);
+        seq_base += (unsigned)gemv_stage<T, Q4, MODEL>(st, cx);
       } else {
         if (st.type == ST_ATTN) {
           AttnBarrier ab;
@@ -1565,9 +1569,9 @@ fsvd_decode_kernel(const Stage* __restrict__ prog_global, const __grid_constant_
         } else {
           if (st.flags & SF_BARRIER) barrier_wait(sync, giveup, target, s, tid);
           trace_mark(trow, 1);
-          if (st.type == ST_EMBED) {
+          if (MODEL && st.type == ST_EMBED) {
             run_embed<T>(st, blockIdx.x * kConsThreads + tid, gridDim.x * kConsThreads);
-          } else if (st.type == ST_ARGMAX) {
+          } else if (MODEL && st.type == ST_ARGMAX) {
             if (blockIdx.x == 0 && warp == 0) run_argmax(st, tid);
           }
         }
