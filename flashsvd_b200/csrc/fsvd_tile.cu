@@ -669,6 +669,11 @@ __global__ void __launch_bounds__(256) exchange_reduce_rows_kernel(const __grid_
 constexpr int kAttnThreads = 128;
 constexpr int kAttnWarps = 4;
 constexpr int kKeyGroup = 8;
+constexpr int kGqKeys = 32;      // keys per warp block of gqa_decode_attn_kernel
+constexpr int kMaxSplit = 64;    // key splits of a sequence at most
+constexpr int kPartPad = 4;      // a record of a split and head: DH sums, running maximum, running sum, padded to 16 bytes
+// Fewest keys of a split: two groups (batch_attn_kernel), one block (gqa_decode_attn_kernel) for each warp.
+constexpr int kBatchSplitKeys = 2 * kAttnWarps * kKeyGroup, kGqSplitKeys = kAttnWarps * kGqKeys;
 
 struct AttnArgs {
   const __nv_bfloat16* q;        // [B, H, Dh], rotated
@@ -676,7 +681,7 @@ struct AttnArgs {
   const __nv_bfloat16* vcache;
   const int* seqlens;
   __nv_bfloat16* out;            // [B, H, Dh]
-  float* part;                   // [B, Hk, nsplit, G, Dh + 2] (acc, m, l)
+  float* part;                   // [B, Hk, nsplit, G, Dh + kPartPad] (acc, m, l)
   int* counters;                 // [B, Hk]
   int B, H, Hk, Dh, S_max, nsplit, seqlen_add, shared_cache;
   float scale;
@@ -688,6 +693,69 @@ struct AttnArgs {
 // Inside a model step the weights are bf16 where they meet the tensor cores.
 template <bool FULL>
 __device__ __forceinline__ float weight(float x) { return FULL ? expf(x) : __expf(x); }
+
+// The splits that a sequence of n positions is cut into: the launch has as many as a full cache takes, a short sequence
+// in it uses fewer, and the CTAs of the others leave at once.  The op alone, caches of 4096 positions, us with all
+// splits and with these: 1 sequence x 32 heads on 16 kv heads, 512 positions 18.4 and 11.1; 8 sequences x 64 heads
+// on 8, 128 positions 15.9 and 11.1; a model step of 8 sequences, 4 layers, 8 positions 428 and 404.
+__device__ __forceinline__ int splits_in_use(int n, int nsplit, int fewest) {
+  return max(1, min(nsplit, (n + fewest - 1) / fewest));
+}
+
+// Merge of the splits of G heads, in split order, by the CTA that arrived last: the weight of every (split, head) once, in
+// shared memory (sh: 2 nsplit G + 16 floats), then each thread sums four output dims over the splits with
+// independent 16-byte loads.  out: [G, DH]
+template <int DH, bool FULL>
+__device__ __forceinline__ void merge_splits(const float* parts, int nsplit, int G, __nv_bfloat16* out, float* sh) {
+  constexpr int rec = DH + kPartPad, U = 8;
+  const int tid = threadIdx.x;
+  float* wgt_s = sh;                       // [nsplit][G] maxima, then weights
+  float* l_s = sh + nsplit * G;            // [nsplit][G] running sums of the splits
+  float* den_s = l_s + nsplit * G;         // [G] sums, [8 + G] maxima
+  for (int i = tid; i < nsplit * G; i += kAttnThreads) {
+    const float2 ml = __ldcg(reinterpret_cast<const float2*>(parts + (size_t)i * rec + DH));
+    wgt_s[i] = ml.x;
+    l_s[i] = ml.y;
+  }
+  __syncthreads();
+  if (tid < G) {
+    float mm = -INFINITY;
+    for (int sp = 0; sp < nsplit; ++sp) mm = fmaxf(mm, wgt_s[sp * G + tid]);
+    den_s[8 + tid] = mm;
+  }
+  __syncthreads();
+  for (int i = tid; i < nsplit * G; i += kAttnThreads) {
+    const float ms = wgt_s[i];
+    wgt_s[i] = ms == -INFINITY ? 0.0f : weight<FULL>(ms - den_s[8 + i % G]);
+  }
+  __syncthreads();
+  if (tid < G) {
+    float den = 0.0f;
+    for (int sp = 0; sp < nsplit; ++sp) den += wgt_s[sp * G + tid] * l_s[sp * G + tid];
+    den_s[tid] = den;
+  }
+  __syncthreads();
+  for (int i = tid; i < G * (DH / 4); i += kAttnThreads) {
+    const int g = i / (DH / 4), d4 = (i - g * (DH / 4)) * 4;
+    float4 num = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (int s0 = 0; s0 < nsplit; s0 += U) {
+      float4 v[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u)   // (past the last split: the last one again, so that U loads are always in flight)
+        v[u] = __ldcg(reinterpret_cast<const float4*>(parts + ((size_t)min(s0 + u, nsplit - 1) * G + g) * rec + d4));
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (s0 + u < nsplit) {
+          const float wg = wgt_s[(s0 + u) * G + g];
+          num.x += wg * v[u].x; num.y += wg * v[u].y; num.z += wg * v[u].z; num.w += wg * v[u].w;
+        }
+    }
+    const float den = den_s[g];
+    uint2 o2 = make_uint2(0u, 0u);
+    if (den > 0.0f) o2 = make_uint2(pack_bf16(num.x / den, num.y / den), pack_bf16(num.z / den, num.w / den));
+    *reinterpret_cast<uint2*>(out + (size_t)g * DH + d4) = o2;
+  }
+}
 
 template <int DPL>
 __device__ __forceinline__ void ld_row(const __nv_bfloat16* row, int lane, float (&f)[DPL]);
@@ -753,7 +821,9 @@ __global__ void __launch_bounds__(kAttnThreads) batch_attn_kernel(const AttnArgs
   idx /= a.nsplit;
   const int hk = idx % a.Hk, b = idx / a.Hk;
   const int n = min(a.seqlens[b] + a.seqlen_add, a.S_max);
-  const int per = (n + a.nsplit - 1) / a.nsplit;
+  const int nsplit = splits_in_use(n, a.nsplit, kBatchSplitKeys);
+  if (split >= nsplit) return;
+  const int per = (n + nsplit - 1) / nsplit;
   const int j0 = min(n, split * per), j1 = min(n, j0 + per);
   const size_t rowstride = (size_t)a.Hk * DH;
   const size_t cbase = ((size_t)b * a.S_max) * rowstride + (size_t)hk * DH;
@@ -836,9 +906,9 @@ __global__ void __launch_bounds__(kAttnThreads) batch_attn_kernel(const AttnArgs
     for (int e = 0; e < DPL; ++e) wacc[warp][g][lane * DPL + e] = acc[g][e];
   }
   __syncthreads();
-  const int nsplit = a.nsplit;
-  const int rec = DH + 2;
-  float* mine = a.part + ((((size_t)b * a.Hk + hk) * nsplit + split) * G) * rec;
+  constexpr int rec = DH + kPartPad;
+  float* const parts = a.part + (((size_t)b * a.Hk + hk) * a.nsplit) * G * rec;
+  float* mine = parts + (size_t)split * G * rec;
   for (int i = tid; i < G * DH; i += kAttnThreads) {
     const int g = i / DH, dd = i - g * DH;
     float mm = -INFINITY;
@@ -872,21 +942,8 @@ __global__ void __launch_bounds__(kAttnThreads) batch_attn_kernel(const AttnArgs
   __syncthreads();
   if (!last_sh) return;
   __threadfence();
-  const float* parts = a.part + (((size_t)b * a.Hk + hk) * nsplit) * G * rec;
-  for (int i = tid; i < G * DH; i += kAttnThreads) {
-    const int g = i / DH, dd = i - g * DH;
-    float mm = -INFINITY;
-    for (int sp = 0; sp < nsplit; ++sp) mm = fmaxf(mm, __ldcg(parts + ((size_t)sp * G + g) * rec + DH));
-    float num = 0.0f, den = 0.0f;
-    for (int sp = 0; sp < nsplit; ++sp) {
-      const float* pr = parts + ((size_t)sp * G + g) * rec;
-      const float ms = __ldcg(pr + DH);
-      const float wgt = ms == -INFINITY ? 0.0f : weight<FULL>(ms - mm);
-      num += wgt * __ldcg(pr + dd);
-      den += wgt * __ldcg(pr + DH + 1);
-    }
-    a.out[((size_t)b * a.H + hk * G + g) * DH + dd] = __float2bfloat16_rn(den > 0.0f ? num / den : 0.0f);
-  }
+  static_assert(kAttnWarps * G * DH >= 2 * kMaxSplit * G + 16);
+  merge_splits<DH, FULL>(parts, nsplit, G, a.out + ((size_t)b * a.H + hk * G) * DH, &wacc[0][0][0]);
 }
 
 // ------------------------------------------------------------------------------- grouped-query decode attention
@@ -898,8 +955,6 @@ __global__ void __launch_bounds__(kAttnThreads) batch_attn_kernel(const AttnArgs
 // rows and 32 value rows into the warp's own shared-memory stage, S = Q K^T, running softmax,
 // O += P V with ldmatrix.trans value fragments (the fragment code of prompt_attn_kernel).  The warps
 // merge in shared memory, the splits of a head in split order by the CTA that arrives last.
-constexpr int kGqKeys = 32;      // keys per warp block
-constexpr int kGqMaxSplit = 64;  // key splits of a sequence at most
 
 template <int DH, bool FULL>
 __global__ void __launch_bounds__(kAttnThreads, 3) gqa_decode_attn_kernel(const AttnArgs a) {
@@ -917,7 +972,9 @@ __global__ void __launch_bounds__(kAttnThreads, 3) gqa_decode_attn_kernel(const 
   idx /= a.nsplit;
   const int hk = idx % a.Hk, b = idx / a.Hk;
   const int n = min(a.seqlens[b] + a.seqlen_add, a.S_max);
-  const int per = ((n + a.nsplit - 1) / a.nsplit + kGqKeys - 1) / kGqKeys * kGqKeys;   // whole blocks per split
+  const int nsplit = splits_in_use(n, a.nsplit, kGqSplitKeys);
+  if (split >= nsplit) return;
+  const int per = ((n + nsplit - 1) / nsplit + kGqKeys - 1) / kGqKeys * kGqKeys;   // whole blocks per split
   const int j0 = min(n, split * per), j1 = min(n, j0 + per);
   const size_t rowstride = (size_t)a.Hk * DH;
   const size_t cbase = ((size_t)b * a.S_max) * rowstride + (size_t)hk * DH;
@@ -1035,9 +1092,8 @@ __global__ void __launch_bounds__(kAttnThreads, 3) gqa_decode_attn_kernel(const 
     }
   }
 
-  // ---- the four warps meet in shared memory (the stages are free): [warp][head][DH + 4]
-  // (DH values, running maximum, running sum; records stay 16-byte aligned)
-  constexpr int rec = DH + 4;
+  // ---- the four warps meet in shared memory (the stages are free): [warp][head] records
+  constexpr int rec = DH + kPartPad;
   __syncthreads();
   float* wpart = reinterpret_cast<float*>(gq_smem);
   if (g < G) {
@@ -1072,8 +1128,8 @@ __global__ void __launch_bounds__(kAttnThreads, 3) gqa_decode_attn_kernel(const 
       }
   }
   __syncthreads();
-  const int nsplit = a.nsplit;
-  float* gpart = a.part + ((((size_t)b * a.Hk + hk) * nsplit + split) * G) * rec;
+  float* const parts = a.part + (((size_t)b * a.Hk + hk) * a.nsplit) * G * rec;
+  float* gpart = parts + (size_t)split * G * rec;
   for (int i = tid; i < G * DH; i += kAttnThreads) {
     const int gg = i / DH, dd = i - gg * DH;
     float mm = -INFINITY;
@@ -1108,51 +1164,7 @@ __global__ void __launch_bounds__(kAttnThreads, 3) gqa_decode_attn_kernel(const 
   __syncthreads();
   if (!last_sh) return;
   __threadfence();
-  // ---- merge of the splits by the last CTA: the weight of every (split, head) once, in shared
-  // memory, then each thread sums four output dims over the splits with independent 16-byte loads
-  const float* parts = a.part + (((size_t)b * a.Hk + hk) * nsplit) * G * rec;
-  float* wgt_s = wpart;                          // [nsplit][G] maxima, then weights (<= 64 x 8)
-  float* den_s = wpart + kGqMaxSplit * 8;        // [G] sums, [8 + G] maxima
-  float* l_s = den_s + 16;                       // [nsplit][G] running sums of the splits
-  for (int i = tid; i < nsplit * G; i += kAttnThreads) {
-    const float2 ml = __ldcg(reinterpret_cast<const float2*>(parts + (size_t)i * rec + DH));
-    wgt_s[i] = ml.x;
-    l_s[i] = ml.y;
-  }
-  __syncthreads();
-  if (tid < G) {
-    float mm = -INFINITY;
-    for (int sp = 0; sp < nsplit; ++sp) mm = fmaxf(mm, wgt_s[sp * G + tid]);
-    den_s[8 + tid] = mm;
-  }
-  __syncthreads();
-  for (int i = tid; i < nsplit * G; i += kAttnThreads) {
-    const float ms = wgt_s[i];
-    wgt_s[i] = ms == -INFINITY ? 0.0f : weight<FULL>(ms - den_s[8 + i % G]);
-  }
-  __syncthreads();
-  if (tid < G) {
-    float den = 0.0f;
-    for (int sp = 0; sp < nsplit; ++sp) den += wgt_s[sp * G + tid] * l_s[sp * G + tid];
-    den_s[tid] = den;
-  }
-  __syncthreads();
-  for (int i = tid; i < G * (DH / 4); i += kAttnThreads) {
-    const int gg = i / (DH / 4), d4 = (i - gg * (DH / 4)) * 4;
-    float4 num = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-#pragma unroll 16
-    for (int sp = 0; sp < nsplit; ++sp) {
-      const float4 v = __ldcg(reinterpret_cast<const float4*>(parts + ((size_t)sp * G + gg) * rec + d4));
-      const float wg = wgt_s[sp * G + gg];
-      num.x += wg * v.x; num.y += wg * v.y; num.z += wg * v.z; num.w += wg * v.w;
-    }
-    const float den = den_s[gg];
-    const float inv = den > 0.0f ? 1.0f / den : 0.0f;
-    uint2 o2;
-    o2.x = pack_bf16(num.x * inv, num.y * inv);
-    o2.y = pack_bf16(num.z * inv, num.w * inv);
-    *reinterpret_cast<uint2*>(a.out + ((size_t)b * a.H + hk * G + gg) * DH + d4) = o2;
-  }
+  merge_splits<DH, FULL>(parts, nsplit, G, a.out + ((size_t)b * a.H + hk * G) * DH, wpart);
 }
 
 }  // namespace fsvd_tile
@@ -1507,7 +1519,7 @@ struct TileWs {
 static int attn_splits(int pairs, int G, int positions, int sms, int most) {
   if (G >= 4) {
     // grouped-query kernel: 3 CTAs per SM, at least one block of 32 keys for each of a CTA's 4 warps
-    most = std::min(most, (positions + 4 * kGqKeys - 1) / (4 * kGqKeys));
+    most = std::min(most, (positions + kGqSplitKeys - 1) / kGqSplitKeys);
     return std::max(1, std::min((3 * sms + pairs - 1) / pairs, most));
   }
   // Three waves of the 8 CTAs of 4 warps that an SM holds, so that the SMs even out: not more than 8 splits
@@ -1515,14 +1527,14 @@ static int attn_splits(int pairs, int G, int positions, int sms, int most) {
   // 8 sequences x 32 heads x 2048 keys 5 splits 2659, 8 2588, 16 2636; 32 sequences 2 splits 4999, 4 4862, 8
   // 4872; 128 sequences x 640 keys 1 split 6494, 2 6658.  A split gets two groups of keys per warp: attention
   // half with 2 heads per kv head, 8 sequences, 300 keys 78 us with one, 74 with two.
-  most = std::max(1, std::min(most, (positions + 2 * kAttnWarps * kKeyGroup - 1) / (2 * kAttnWarps * kKeyGroup)));
+  most = std::max(1, std::min(most, (positions + kBatchSplitKeys - 1) / kBatchSplitKeys));
   const int wave = (8 * sms + pairs - 1) / pairs;
   return std::min(most, std::min((24 * sms + pairs - 1) / pairs, std::max(8, wave)));
 }
 static int attn_nsplit(const fsvd_dims& D, int sms) {
   if (D.rows_are_positions || D.Hk < 1) return 1;   // prompt pass: row blocks share the cache rows instead
   const int G = D.H / D.Hk;
-  return attn_splits(D.B * D.Hk, G, D.S_max, sms, G >= 4 ? kGqMaxSplit : 16);
+  return attn_splits(D.B * D.Hk, G, D.S_max, sms, G >= 4 ? kMaxSplit : 16);
 }
 static int imax(int a, int b) { return a > b ? a : b; }
 static TileWs tile_layout(const fsvd_dims& D, int sms) {
@@ -1540,7 +1552,7 @@ static TileWs tile_layout(const fsvd_dims& D, int sms) {
   L.mid = o;       o += al256((size_t)B * D.d * 2);
   L.hact = o;      o += al256((size_t)B * D.I * 2);
   L.nsplit = attn_nsplit(D, sms);
-  L.apart = o;     o += al256((size_t)B * D.Hk * L.nsplit * (D.H / imax(D.Hk, 1)) * (D.Dh + 4) * 4);
+  L.apart = o;     o += al256((size_t)B * D.Hk * L.nsplit * (D.H / imax(D.Hk, 1)) * (D.Dh + kPartPad) * 4);
   L.total = o;
   return L;
 }
@@ -1825,8 +1837,7 @@ int fsvd_tile_flash_decode(const void* q, const void* k_cache, const void* v_cac
   at.seqlens = cache_seqlens; at.out = reinterpret_cast<__nv_bfloat16*>(out);
   at.part = part; at.counters = counters;
   at.B = B; at.H = H; at.Hk = Hk; at.Dh = Dh; at.S_max = S_max; at.seqlen_add = seqlen_add; at.scale = scale;
-  // a split's record is Dh + 4 floats per head at most
-  const int fits = (int)std::min<size_t>(part_floats / ((size_t)B * H * (Dh + 4)), kGqMaxSplit);
+  const int fits = (int)std::min<size_t>(part_floats / ((size_t)B * H * (Dh + kPartPad)), kMaxSplit);
   at.nsplit = attn_splits(B * Hk, H / Hk, S_max, g_sms, std::max(1, fits));
   return launch_attn(at, (cudaStream_t)stream, true);
 }
