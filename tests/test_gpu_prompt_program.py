@@ -168,3 +168,39 @@ def test_prompts_in_captured_graphs(B):
         first.close()
         tokenwise.close()
     ref.close()
+
+
+@pytest.mark.parametrize("shape,B,L", [(O.TINY, 1, 2049), (O.TINY_GQA, 1, 4100), (O.TINY_GQA, 3, 700), (O.TINY, 128, 17), (O.TINY_GQA, 128, 33)])
+def test_prompts_of_several_passes(shape, B, L):
+    """More than 2048 rows in one call (a pass that is not the last one, the short last one, keys of an earlier
+    pass read by a later one), every sequence at a start of its own with keys and values already there:
+    against the same prompt token by token.  Tolerance as above: two orders of addition over two layers and the head."""
+    start = [5 + 3 * (b % 4) for b in range(B)]
+    S_max = L + 20
+    w = O.make_model_weights(shape, seed=9, dtype=torch.bfloat16)
+    gen = torch.Generator().manual_seed(L)
+    prompt = torch.randint(0, shape.vocab, (B, L), generator=gen, dtype=torch.int32).cuda()
+    past = torch.randn(2, shape.n_layers, B, max(start), shape.Hk, shape.Dh, generator=gen).to(torch.bfloat16).cuda()
+    engines = []
+    for chunk in (None, 1):
+        eng = _engine(shape, w, B, S_max, prefill_chunk=chunk)
+        for li in range(shape.n_layers):
+            eng.key_cache[li][:, :max(start)], eng.value_cache[li][:, :max(start)] = past[0, li], past[1, li]
+        eng.seqlens.copy_(torch.tensor(start, dtype=torch.int32))
+        before = eng.step_counter.item()
+        eng.prefill(prompt)
+        torch.cuda.synchronize()
+        assert eng.status() == 0
+        assert eng.seqlens.tolist() == [s + L for s in start]
+        assert eng.step_counter.item() == before + (1 if chunk is None else L)
+        assert torch.equal(eng.tokens.long(), eng.logits.argmax(dim=1))
+        engines.append(eng)
+    one, ref = engines
+    assert rel_linf(one.logits, ref.logits) <= 4e-2
+    for li in range(shape.n_layers):
+        for a, b in ((one.key_cache[li], ref.key_cache[li]), (one.value_cache[li], ref.value_cache[li])):
+            assert rel_linf(a, b) <= 4e-2
+            for s in range(B):   # nothing outside the prompt's rows is touched
+                assert torch.equal(a[s, :start[s]], b[s, :start[s]]) and not bool(a[s, start[s] + L:].any())
+    for eng in engines:
+        eng.close()
