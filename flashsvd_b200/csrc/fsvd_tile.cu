@@ -1,9 +1,10 @@
-// Decode for batches of 9..128 sequences (bf16): the factor products as tiled GEMMs on the 5th
+// Decode for batches of 5..128 sequences (bf16): the factor products as tiled GEMMs on the 5th
 // generation tensor cores.
 //
 // With more than 8 activation rows per factor row the 16 x 8 register tiles of the persistent
 // interpreter (fsvd_kernel.cuh) no longer fit the batch; here a factor product is
-//     D[128 factor rows, N batch columns] = W[128, K] . X[N, K]^T        (N = batch rounded up to 16)
+//     D[128 factor rows, N batch columns] = W[128, K] . X[N, K]^T
+// (N = batch rounded up to 16; from 65 sequences on two CTAs may take half of it each)
 // issued as tcgen05.mma (cta_group::1, kind::f16, M = 128) by one thread per CTA, with both operands
 // read from shared memory (128-byte swizzled, K-major, filled by TMA) and the fp32 accumulator in
 // tensor memory.  The work is still bound by the factor stream from HBM (each factor byte is used
@@ -14,7 +15,7 @@
 //     no partial sum goes through global memory and the result does not depend on timing;
 //   * a ring of NS stages {W tile 16 KB, (second W tile), X tile(s)}: three threads issue the TMA copies
 //     as slots free up, thread 32 issues the MMAs as slots fill and releases a slot with
-//     tcgen05.commit, all four warps read the accumulator back with tcgen05.ld for the epilogue;
+//     tcgen05.commit, all eight warps read the accumulator back with tcgen05.ld for the epilogue;
 //   * epilogues: store / residual / SwiGLU (two accumulators) / RoPE + q buffer / RoPE + key cache /
 //     value cache, with the rounding points of the PyTorch low-rank path (every nn.Linear output
 //     rounded to bf16), the same as the interpreter's.
@@ -1703,7 +1704,7 @@ static cudaError_t launch_attn_g(const AttnArgs& at, cudaStream_t st) {
   }
 }
 static PaArgs prompt_args(const AttnArgs& at) {
-  PaArgs pa;
+  PaArgs pa;   // (a row sees the keys up to its own position: seqlen_add is 1 on this route)
   pa.q = at.q; pa.kcache = at.kcache; pa.vcache = at.vcache; pa.rowpos = at.seqlens; pa.rowseq = nullptr; pa.out = at.out;
   pa.L = at.B; pa.H = at.H; pa.Hk = at.Hk; pa.S_max = at.S_max;
   pa.scale_log2 = at.scale * 1.4426950408889634f;

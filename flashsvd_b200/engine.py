@@ -8,7 +8,6 @@ Token ids and sequence lengths stay on the device between steps, which removes t
 from __future__ import annotations
 
 import ctypes as C
-from typing import Optional
 
 import torch
 
@@ -93,9 +92,10 @@ class DecodeEngine:
         self.handle = handle
         self.max_steps = int(max_steps)
         self._pos_bound = 0   # host-side upper bound of the cache positions in use
-        # Prompt pass of a single sequence: a second program over the same weights and caches takes
+        # Prompt of a single fp32 or int4 sequence: a second program over the same weights and caches takes
         # `prefill_chunk` consecutive prompt positions per launch (rows_are_positions of fsvd_dims);
-        # it is created on the first prompt that is long enough.
+        # it is created on the first prompt that is long enough.  For bf16, where the prompt program below takes
+        # every prompt, `prefill_chunk=1` asks for token by token and any other value means the program.
         cmax = 4 if dtype == torch.float32 else 8
         self.prefill_chunk = (cmax if prefill_chunk is None else max(1, min(int(prefill_chunk), cmax))) \
             if self.B == 1 else 1
@@ -104,7 +104,6 @@ class DecodeEngine:
         self.prefill_tile = 128 if (dtype == torch.bfloat16 and not q4 and prefill_chunk != 1
                                     and self.dims.Rg == self.dims.Ru) else 0
         self._layer_array, self._model_args = arr, (embed, final_norm, lm_head)
-        self._chunk_handle = None
         self._chunks: dict = {}
         ptrs = [C.c_void_p() for _ in range(6)]
         check(self.lib.fsvd_model_buffers(self.handle, *[C.byref(p) for p in ptrs]))
@@ -161,10 +160,10 @@ class DecodeEngine:
         self.step_counter.zero_()
         self._pos_bound = 0
 
-    def _chunk_model(self, rows: Optional[int] = None):
-        """The program that takes `rows` (default `prefill_chunk`) prompt positions of the one
-        sequence per launch; returns (handle, tokens view, seqlens view)."""
-        rows = int(self.prefill_chunk if rows is None else rows)
+    def _chunk_model(self):
+        """The program that takes `prefill_chunk` prompt positions of the one sequence per launch; returns
+        (handle, tokens view, seqlens view)."""
+        rows = self.prefill_chunk
         hit = self._chunks.get(rows)
         if hit is None:
             d = self.dims
@@ -181,8 +180,6 @@ class DecodeEngine:
             hit = (handle, _from_ptr(ptrs[0].value, (rows,), torch.int32, self.device),
                    _from_ptr(ptrs[1].value, (rows,), torch.int32, self.device), dims)
             self._chunks[rows] = hit
-            if rows == self.prefill_chunk:
-                self._chunk_handle, self._chunk_tokens, self._chunk_seqlens, self._chunk_dims = hit
         return hit[:3]
 
     def _prompt_program(self):
@@ -224,7 +221,7 @@ class DecodeEngine:
             check(self.lib.fsvd_prompt_run(handle, prompt.data_ptr(), L, L, stream))
             return
         if self.B == 1 and L > Cn > 1:
-            handle, tokens, seqlens = self._chunk_model(Cn)
+            handle, tokens, seqlens = self._chunk_model()
             offs = torch.arange(Cn, device=self.device, dtype=torch.int32)
             while L - t0 > Cn:
                 tokens.copy_(prompt[0, t0:t0 + Cn])
@@ -259,7 +256,6 @@ class DecodeEngine:
             if hit[0].value:
                 self.lib.fsvd_model_destroy(hit[0])
         self._chunks = {}
-        self._chunk_handle = None
         if getattr(self, "handle", None) is not None and self.handle.value:
             self.lib.fsvd_model_destroy(self.handle)
             self.handle = C.c_void_p()

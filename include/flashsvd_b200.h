@@ -215,7 +215,8 @@ int fsvd_qkv_rope_append(const void* x, const void* norm_w, float eps, const voi
 /* out[B,H,Dh] = softmax(q·K^T * scale)·V over the first cache_seqlens[b] + seqlen_add cached
  * positions (GQA by head grouping), split over the keys and combined in split order.  Replaces
  * the attention half of flash_attn_with_kvcache (runtime/attn/decode_registry.py:177-211);
- * scale <= 0 selects 1/sqrt(Dh). */
+ * scale <= 0 selects 1/sqrt(Dh).  The softmax weights are fp32 (bf16 tensors too).  bf16 tensors that all start on
+ * 16-byte boundaries take the faster kernels. */
 int fsvd_flash_decode(const void* q, const void* k_cache, const void* v_cache,
                       const int* cache_seqlens, int seqlen_add, void* out,
                       int B, int H, int Hk, int Dh, int S_max, float scale, int dtype,
@@ -224,7 +225,8 @@ int fsvd_flash_decode(const void* q, const void* k_cache, const void* v_cache,
 /* One whole decoder layer for one new token per sequence, one launch:
  * x_out = h + mlp(rms(h)), h = x_in + attn(rms(x_in)); the layer's caches receive the new
  * token at position cache_seqlens[b].  Replaces transformers' LlamaDecoderLayer.forward as the
- * reference drives it from utils/evaluator.py:69-78 in mode="flashsvd". */
+ * reference drives it from utils/evaluator.py:69-78 in mode="flashsvd".  x_in may start at any
+ * address for batches of the tiled path (bf16, 5..128); else on a 16-byte boundary. */
 int fsvd_decode_layer(const fsvd_dims* dims, const fsvd_layer* layer, const void* cos_tab,
                       const void* sin_tab, const int* cache_seqlens, const void* x_in, void* x_out,
                       void* ws, size_t ws_bytes, void* stream);
