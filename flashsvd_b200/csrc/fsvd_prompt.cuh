@@ -322,16 +322,19 @@ __global__ void __launch_bounds__(kPgThreads, 1) prompt_gemm_kernel(const __grid
 // cp.async one block ahead and serve all of them.  S = Q K^T and O += P V on mma.sync m16n8k16 (bf16,
 // fp32 accumulation) with fragments taken by ldmatrix; running softmax in base 2; only blocks that reach
 // past a query's own position are masked.  Query blocks with the longest range start first.
-// The softmax weights of the rows from full_from on meet the value rows with all their 24 bits, as three bf16
-// numbers; those of the rows before are rounded to bf16.  Full are the prompts of several sequences, short
-// blocks of rows and the last kFullRows positions of one sequence (they decide the first token): where a
-// feed token by token or in a few rows has fp32 weights.  The attention of a long prompt is bound by mma.sync:
-// 2041 positions through 4 layers of 32 heads of 128 take 2.85 ms with no full row, 2.90 like this, 3.12 with
-// every row full; six prompts of 190 (all rows full) 1.53 and 1.56 ms.
+//
+// Softmax weights meet the value rows rounded to bf16, or with all their 24 bits as three bf16 numbers (FULL), so that
+// a prompt has no fewer bits than a feed token by token, whose kernels have fp32 weights up to 4 sequences or with 1 or
+// 2 heads per kv head.  All rows of several such sequences are FULL.  A single sequence has its last kFullRows positions FULL
+// (they decide the first token), by CTAs of their own in front of the others: 16 query vectors, the key blocks dealt
+// out to the four warps, which are through long before a block of 64 with as many keys.  The earlier rows are bound
+// by mma.sync: 2041 positions through 4 layers of 32 heads of 128 take 2.80 ms with no FULL row, 2.77 like this, 2.90 with
+// the last block of 64 rows FULL and 3.12 with all of them; 4 prompts of 180 (all FULL) 1.37 and 1.40 ms.
 constexpr int kPaWarps = 4;
 constexpr int kPaSlots = 16 * kPaWarps;
 constexpr int kPaKeys = 64;
 constexpr int kFullRows = 16;
+constexpr int kPaTailSlots = 16, kPaTailKeys = 32;   // query vectors of a CTA, keys of a warp's block
 
 struct PaArgs {
   const __nv_bfloat16* q;        // [rows, H, Dh], rotated
@@ -341,7 +344,7 @@ struct PaArgs {
   const int* rowseq;             // [rows] cache row, or null: cache row 0
   __nv_bfloat16* out;            // [rows, H, Dh]
   int L, H, Hk, S_max;           // rows per sequence
-  int full_from;                 // rows of a sequence from here on: 24-bit weights
+  int full_from;                 // rows of a sequence from here on go to the CTAs of 16 query vectors (L: none)
   float scale_log2;              // softmax scale x log2(e)
 };
 
@@ -361,9 +364,9 @@ __device__ __forceinline__ void prompt_attn_rows(const PaArgs& a, unsigned char*
   for (int i = 0; i < 2; ++i) {
     const int m = m0 + 8 * i;
     const int r = r0 + m / G;
-    rowq[i] = seq0 + min(r, a.L - 1);
+    rowq[i] = seq0 + min(r, rlast);
     headq[i] = hk * G + m % G;
-    nl[i] = r < a.L ? min(nfirst + m / G, a.S_max) : 0;
+    nl[i] = r <= rlast ? min(nfirst + m / G, a.S_max) : 0;
   }
   uint32_t qa[KS][4];
 #pragma unroll
@@ -516,16 +519,187 @@ __device__ __forceinline__ void prompt_attn_rows(const PaArgs& a, unsigned char*
     }
 }
 
+// Rows r0 .. rlast (at most 16 / G of them), the keys in blocks of 32 dealt out to the warps, which merge at the end.
 template <int DH>
+__device__ __forceinline__ void prompt_attn_tail(const PaArgs& a, unsigned char* pa_smem, int seq0, int r0, int rlast) {
+  constexpr int STRIDE = DH * 2 + 16, KS = DH / 16, NT = kPaTailKeys / 8, DT = DH / 8, PIECES = DH / 8;
+  constexpr int rec = DH + kPartPad;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int G = a.H / a.Hk, hk = blockIdx.y;
+  const int nfirst = a.rowpos[seq0 + r0] + 1, nmax = min(a.rowpos[seq0 + rlast] + 1, a.S_max);
+  int nl[2];
+  uint32_t qa[KS][4];
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int m = g + 8 * i, r = r0 + m / G;
+    nl[i] = r <= rlast ? min(nfirst + m / G, a.S_max) : 0;
+    const __nv_bfloat16* qp = a.q + ((size_t)(seq0 + min(r, rlast)) * a.H + hk * G + m % G) * DH + 2 * t;
+#pragma unroll
+    for (int ks = 0; ks < KS; ++ks) {
+      qa[ks][i] = *reinterpret_cast<const uint32_t*>(qp + ks * 16);
+      qa[ks][2 + i] = *reinterpret_cast<const uint32_t*>(qp + ks * 16 + 8);
+    }
+  }
+  float o[DT][4], mrow[2] = {-INFINITY, -INFINITY}, lrow[2] = {0.0f, 0.0f};   // maxima in units of log2
+#pragma unroll
+  for (int d = 0; d < DT; ++d) o[d][0] = o[d][1] = o[d][2] = o[d][3] = 0.0f;
+  const size_t rowstride = (size_t)a.Hk * DH;
+  const size_t cbase = (size_t)(a.rowseq ? a.rowseq[seq0] : 0) * a.S_max * rowstride + (size_t)hk * DH;
+  const __nv_bfloat16* kbase = a.kcache + cbase;
+  const __nv_bfloat16* vbase = a.vcache + cbase;
+  const uint32_t ks_s = smem_u32(pa_smem) + (uint32_t)(warp * 2 * kPaTailKeys * STRIDE), vs_s = ks_s + kPaTailKeys * STRIDE;
+
+  for (int k0 = warp * kPaTailKeys; k0 < nmax; k0 += kPaWarps * kPaTailKeys) {
+    __syncwarp();
+    for (int i = lane; i < kPaTailKeys * PIECES; i += 32) {
+      const int r = i / PIECES, c = i - r * PIECES;
+      const size_t src = (size_t)min(k0 + r, nmax - 1) * rowstride + (size_t)c * 8;   // past the end: masked below
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(ks_s + r * STRIDE + c * 16), "l"(kbase + src) : "memory");
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(vs_s + r * STRIDE + c * 16), "l"(vbase + src) : "memory");
+    }
+    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+    __syncwarp();
+    float sc[NT][4];
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt) sc[nt][0] = sc[nt][1] = sc[nt][2] = sc[nt][3] = 0.0f;
+    const uint32_t kaddr = ks_s + (uint32_t)(((lane & 7) + ((lane >> 4) & 1) * 8) * STRIDE + ((lane >> 3) & 1) * 16);
+#pragma unroll
+    for (int j = 0; j < NT / 2; ++j) {
+#pragma unroll
+      for (int ks = 0; ks < KS; ++ks) {
+        uint32_t b0, b1, b2, b3;
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                     : "=r"(b0), "=r"(b1), "=r"(b2), "=r"(b3) : "r"(kaddr + (uint32_t)(j * 16 * STRIDE + ks * 32)));
+        mma_bf16_16816(sc[2 * j], qa[ks][0], qa[ks][1], qa[ks][2], qa[ks][3], b0, b1);
+        mma_bf16_16816(sc[2 * j + 1], qa[ks][0], qa[ks][1], qa[ks][2], qa[ks][3], b2, b3);
+      }
+    }
+    float mx[2] = {-INFINITY, -INFINITY};
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        sc[nt][e] = k0 + nt * 8 + 2 * t + (e & 1) < nl[e >> 1] ? sc[nt][e] * a.scale_log2 : -INFINITY;
+        mx[e >> 1] = fmaxf(mx[e >> 1], sc[nt][e]);
+      }
+    float ps[2] = {0.0f, 0.0f}, mref[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      mx[i] = fmaxf(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], 1));
+      mx[i] = fmaxf(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], 2));
+      const float mn = fmaxf(mrow[i], mx[i]);
+      mref[i] = mn == -INFINITY ? 0.0f : mn;   // nothing visible yet: every weight is 0
+      const float corr = exp2f(mrow[i] - mref[i]);
+      mrow[i] = mn;
+      lrow[i] *= corr;
+#pragma unroll
+      for (int d = 0; d < DT; ++d) {
+        o[d][2 * i] *= corr;
+        o[d][2 * i + 1] *= corr;
+      }
+    }
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        sc[nt][e] = exp2f(sc[nt][e] - mref[e >> 1]);
+        ps[e >> 1] += sc[nt][e];
+      }
+    lrow[0] += ps[0];   // (summed over the row's four lanes at the end)
+    lrow[1] += ps[1];
+#pragma unroll
+    for (int kk = 0; kk < kPaTailKeys / 16; ++kk) {
+      uint32_t p[3][4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        split_bf16(sc[2 * kk + (i >> 1)][2 * (i & 1)], sc[2 * kk + (i >> 1)][2 * (i & 1) + 1], p[0][i], p[1][i], p[2][i]);
+      const uint32_t vaddr = vs_s + (uint32_t)((kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * STRIDE + ((lane >> 4) & 1) * 16);
+#pragma unroll
+      for (int j = 0; j < DT / 2; ++j) {
+        uint32_t b0, b1, b2, b3;
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                     : "=r"(b0), "=r"(b1), "=r"(b2), "=r"(b3) : "r"(vaddr + j * 32));
+#pragma unroll
+        for (int w = 2; w >= 0; --w) {
+          mma_bf16_16816(o[2 * j], p[w][0], p[w][1], p[w][2], p[w][3], b0, b1);
+          mma_bf16_16816(o[2 * j + 1], p[w][0], p[w][1], p[w][2], p[w][3], b2, b3);
+        }
+      }
+    }
+  }
+  // ---- the warps meet in shared memory (the stages are free): [warp][query vector] records
+  __syncthreads();
+  float* const recs = reinterpret_cast<float*>(pa_smem);
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    lrow[i] += __shfl_xor_sync(0xffffffffu, lrow[i], 1);
+    lrow[i] += __shfl_xor_sync(0xffffffffu, lrow[i], 2);
+    float* mine = recs + (warp * kPaTailSlots + g + 8 * i) * rec;
+    bool none = false;   // "no number" among this thread's sums
+#pragma unroll
+    for (int d = 0; d < DT; ++d) {
+      mine[d * 8 + 2 * t] = o[d][2 * i];
+      mine[d * 8 + 2 * t + 1] = o[d][2 * i + 1];
+      none |= o[d][2 * i] != o[d][2 * i] || o[d][2 * i + 1] != o[d][2 * i + 1];
+    }
+    if (t == 0) {
+      mine[DH] = mrow[i];
+      mine[DH + 1] = lrow[i];
+    }
+    unsigned again = __ballot_sync(0xffffffffu, nl[i] > 0 && none);
+    __syncwarp();
+#pragma unroll 1
+    for (int m = 8 * i; again; ++m, again >>= 4)
+      if (again & 15u) {
+        const int r = r0 + m / G;
+        float acc[DH / 32], mm, ll;
+        attn_one_row<DH>(a.q + ((size_t)(seq0 + r) * a.H + hk * G + m % G) * DH, kbase, vbase, rowstride, warp * kPaTailKeys,
+                         min(nfirst + r - r0, a.S_max), kPaTailKeys, kPaWarps * kPaTailKeys, a.scale_log2 * 0.6931471805599453f, acc,
+                         &mm, &ll);
+        float* to = recs + (warp * kPaTailSlots + m) * rec;
+#pragma unroll
+        for (int e = 0; e < DH / 32; ++e) to[lane * (DH / 32) + e] = acc[e];
+        if (lane == 0) {
+          to[DH] = mm * 1.4426950408889634f;
+          to[DH + 1] = ll;
+        }
+      }
+  }
+  __syncthreads();
+  for (int i = tid; i < (rlast - r0 + 1) * G * (DH / 2); i += kPaWarps * 32) {
+    const int m = i / (DH / 2), d = 2 * (i - m * (DH / 2));
+    float mm = -INFINITY;
+#pragma unroll
+    for (int w = 0; w < kPaWarps; ++w) mm = fmaxf(mm, recs[(w * kPaTailSlots + m) * rec + DH]);
+    float x = 0.0f, y = 0.0f, den = 0.0f;
+#pragma unroll
+    for (int w = 0; w < kPaWarps; ++w) {
+      const float* pr = recs + (w * kPaTailSlots + m) * rec;
+      const float wgt = pr[DH] == -INFINITY ? 0.0f : exp2f(pr[DH] - mm);
+      x += wgt * pr[d];
+      y += wgt * pr[d + 1];
+      den += wgt * pr[DH + 1];
+    }
+    const float inv = den > 0.0f ? 1.0f / den : 0.0f;
+    *reinterpret_cast<uint32_t*>(a.out + ((size_t)(seq0 + r0 + m / G) * a.H + hk * G + m % G) * DH + d) = pack_bf16(x * inv, y * inv);
+  }
+}
+
+template <int DH, bool FULL>
 __global__ void __launch_bounds__(kPaWarps * 32, DH == 64 ? 4 : 3) prompt_attn_kernel(const PaArgs a) {
   extern __shared__ __align__(16) unsigned char pa_smem[];
   pdl_launch_dependents();
   pdl_wait();
-  const int rpb = kPaSlots / (a.H / a.Hk);            // positions per CTA
-  const int r0 = (gridDim.x - 1 - blockIdx.x) * rpb;  // first row of the CTA, inside the sequence
-  const int rlast = min(r0 + rpb, a.L) - 1;
-  if (rlast >= a.full_from) prompt_attn_rows<DH, true>(a, pa_smem, blockIdx.z * a.L, r0, rlast);
-  else prompt_attn_rows<DH, false>(a, pa_smem, blockIdx.z * a.L, r0, rlast);
+  const int G = a.H / a.Hk, seq0 = blockIdx.z * a.L;
+  const int tpos = kPaTailSlots / G, ntail = FULL ? 0 : (a.L - a.full_from + tpos - 1) / tpos;
+  if ((int)blockIdx.x < ntail) {
+    const int r0 = a.full_from + (ntail - 1 - (int)blockIdx.x) * tpos;
+    prompt_attn_tail<DH>(a, pa_smem, seq0, r0, min(r0 + tpos, a.L) - 1);
+    return;
+  }
+  const int rpb = kPaSlots / G;                                   // positions per CTA
+  const int r0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * rpb;    // first row of the CTA, inside the sequence
+  prompt_attn_rows<DH, FULL>(a, pa_smem, seq0, r0, min(r0 + rpb, a.full_from) - 1);
 }
 
 }  // namespace fsvd_tile

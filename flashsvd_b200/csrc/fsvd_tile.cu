@@ -1669,21 +1669,25 @@ static int plan_layer(LayerPlan& lp, const fsvd_dims& D, const fsvd_layer& Lw, c
   return 0;
 }
 
-template <int DH>
+template <int DH, bool FULL>
 static cudaError_t launch_prompt_attn(const PaArgs& pa, int nseq, cudaStream_t st) {
   constexpr int smem = 4 * kPaKeys * (DH * 2 + 16);
+  static_assert(kPaWarps * kPaTailSlots * (DH + kPartPad) * 4 <= smem && kPaWarps * 2 * kPaTailKeys * (DH * 2 + 16) <= smem);
   static SmemLimit limit;
-  const cudaError_t e = limit.raise(prompt_attn_kernel<DH>, smem);
+  const cudaError_t e = limit.raise(prompt_attn_kernel<DH, FULL>, smem);
   if (e != cudaSuccess) return e;
-  const int rpb = kPaSlots / (pa.H / pa.Hk);
-  return launch_pdl(prompt_attn_kernel<DH>, dim3((unsigned)((pa.L + rpb - 1) / rpb), (unsigned)pa.Hk, (unsigned)nseq),
-                    dim3(kPaWarps * 32), (size_t)smem, st, pa);
+  const int G = pa.H / pa.Hk, rpb = kPaSlots / G, tpos = kPaTailSlots / G;
+  const int ctas = (pa.full_from + rpb - 1) / rpb + (FULL ? 0 : (pa.L - pa.full_from + tpos - 1) / tpos);
+  return launch_pdl(prompt_attn_kernel<DH, FULL>, dim3((unsigned)ctas, (unsigned)pa.Hk, (unsigned)nseq), dim3(kPaWarps * 32), (size_t)smem,
+                    st, pa);
 }
 // rows of nseq sequences, L consecutive positions each
 static int launch_prompt_attn(PaArgs pa, int Dh, int nseq, cudaStream_t st) {
-  pa.full_from = nseq > 1 ? 0 : pa.L - kFullRows;
-  if ((Dh == 128 ? launch_prompt_attn<128>(pa, nseq, st) : launch_prompt_attn<64>(pa, nseq, st)) != cudaSuccess)
-    return launch_failed("attention kernel launch failed");
+  const bool full = nseq > 1 && (nseq <= 4 || pa.H / pa.Hk < 4);
+  pa.full_from = nseq > 1 ? pa.L : std::max(0, pa.L - kFullRows);
+  const cudaError_t e = Dh == 128 ? (full ? launch_prompt_attn<128, true>(pa, nseq, st) : launch_prompt_attn<128, false>(pa, nseq, st))
+                                  : (full ? launch_prompt_attn<64, true>(pa, nseq, st) : launch_prompt_attn<64, false>(pa, nseq, st));
+  if (e != cudaSuccess) return launch_failed("attention kernel launch failed");
   fsvd_tile_count_launch();
   return 0;
 }

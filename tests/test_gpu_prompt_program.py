@@ -204,3 +204,35 @@ def test_prompts_of_several_passes(shape, B, L):
                 assert torch.equal(a[s, :start[s]], b[s, :start[s]]) and not bool(a[s, start[s] + L:].any())
     for eng in engines:
         eng.close()
+
+
+@pytest.mark.parametrize("shape,B,L,at", [(O.TINY, 1, 60, 30), (O.TINY, 1, 60, 55), (O.TINY, 2, 60, 30), (O.TINY_GQA, 6, 60, 30),
+                                          (WIDE_HEADS, 3, 20, 9)])
+def test_an_infinite_value_stays_at_its_position(shape, B, L, at):
+    """One token of sequence 0 has infinite values in the first layer: the rows before it, and the other
+    sequences, have the same keys and values in the second layer as without it."""
+    dtype = torch.bfloat16
+    w = O.make_model_weights(shape, seed=12, dtype=dtype)
+    w["embed"][:, 5] = 0.0
+    w["embed"][7, 5] = 4.0                      # token 7 alone has this dimension ...
+    first = w["layers"][0]
+    first["v_v"][0] = 0.0
+    first["v_v"][0, 5] = 1.0                    # ... which is rank 0 of the values
+    first["v_u"][:, 0] = 3e38
+    prompt = torch.randint(8, shape.vocab, (B, L), generator=torch.Generator().manual_seed(B), dtype=torch.int32).cuda()
+    bad = prompt.clone()
+    bad[0, at] = 7
+    states = []
+    for ids in (prompt, bad):
+        eng = _engine(shape, w, B, L + 4)
+        eng.prefill(ids)
+        torch.cuda.synchronize()
+        assert eng.status() == 0
+        states.append([t.clone() for t in (eng.value_cache[0], eng.key_cache[1], eng.value_cache[1])])
+        eng.close()
+    (v0, *clean), (v0_bad, *got) = states
+    assert bool(v0.isfinite().all()) and bool(v0_bad[0, at].isinf().all())
+    for a, b in zip(got, clean):
+        assert rel_linf(a[0, :at], b[0, :at]) <= 2e-2
+        assert torch.equal(a[1:], b[1:])
+        assert not bool(a[0, at].isfinite().any())

@@ -75,19 +75,21 @@ def test_prompt_rows(H, Hk, Dh, B):
     got = out.double().cpu()[-16:].view(-1, H, Dh)
     n = Dh - 1                               # (the last dimension of the last head holds the residual)
     assert bool(((got - ref).abs() <= tol)[..., :n].all())
-    # An infinite value at a later position (row B - 2's, in dimensions 7 and 8) is nothing to the rows before it, whatever
-    # tile they share.  Their values: tolerance as above where the weights have 24 bits, else 2^-8 of |p v1| more.
-    xin[B - 2] = 0.0
-    xin[B - 2, d - 2] = 2.0 ** -20
+    # An infinite value at a later position (in dimensions 7 and 8) is nothing to the rows before it, whatever tile they
+    # share.  Their values: tolerance as above where the weights have 24 bits, else 2^-8 of |p v1| more.
     qkv_v[16, d - 2] = 1.0
     pk["v_u"][7::Dh, 0], pk["v_u"][8::Dh, 0] = 3e38, -3e38
-    run()
-    assert bool(pk["v_cache"][0, ctx + B - 2, :, 7:9].isinf().all())
-    got = out.double().cpu()[:B - 2].view(-1, H, Dh)
-    wide = torch.full((B - 2, 1, 1), 2.0 ** -8).double()
-    wide[max(0, B - 16):] = 0.0
-    assert bool(((got - ref).abs() <= tol + wide * 512)[..., :n].all())
-    assert not bool(out[B - 2:].view(-1, H, Dh)[..., 7].isfinite().any())
+    for bad in (B - 2, B // 2):
+        xin[:] = 0.0
+        xin[:, d - 1] = 2.0 ** -20
+        xin[bad, d - 1], xin[bad, d - 2] = 0.0, 2.0 ** -20
+        run()
+        assert bool(pk["v_cache"][0, ctx + bad, :, 7:9].isinf().all())
+        got = out.double().cpu()[:bad].view(-1, H, Dh)
+        wide = torch.full((bad, 1, 1), 2.0 ** -8).double()
+        wide[max(0, B - 16):] = 0.0
+        assert bool(((got - ref).abs() <= tol + wide * 512)[..., :n].all())
+        assert not bool(out[bad:].view(-1, H, Dh)[..., 7].isfinite().any())
 
 
 @pytest.mark.parametrize("n", [3, 70, 1200])
