@@ -2015,18 +2015,20 @@ int fsvd_tile_model_destroy(fsvd_tile_model* m) {
   return 0;
 }
 
-// Zeroes fresh device memory before any stream can use it.  (cudaMemset goes to the default stream and returns
-// at once; a pass on a non-blocking stream would not wait for it.  A stream of its own does not wait for
-// what the default stream has queued.)
-static cudaError_t clear_now(void* p, size_t bytes) {
-  cudaStream_t st;
-  cudaError_t ce = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
-  if (ce != cudaSuccess) return ce;
-  ce = cudaMemsetAsync(p, 0, bytes, st);
-  if (ce == cudaSuccess) ce = cudaStreamSynchronize(st);
-  cudaStreamDestroy(st);
-  return ce;
-}
+// A stream on which fresh device memory is zeroed before any other stream can use it.  (cudaMemset goes to the
+// default stream and returns at once: a launch on a non-blocking stream would not wait for it.  A stream of
+// its own does not wait for what the default stream has queued.)
+struct SideStream {
+  cudaStream_t st = nullptr;
+  cudaError_t clear(void* p, size_t bytes) {
+    cudaError_t ce = st ? cudaSuccess : cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+    return ce != cudaSuccess ? ce : cudaMemsetAsync(p, 0, bytes, st);
+  }
+  cudaError_t wait() { return cudaStreamSynchronize(st); }
+  ~SideStream() {
+    if (st) cudaStreamDestroy(st);
+  }
+};
 
 int fsvd_tile_model_create(const fsvd_dims* dims, const fsvd_layer* layers, const void* embed, const void* final_norm_w,
                            const void* lm_head, const void* cos_tab, const void* sin_tab, int max_steps, long long wait_limit,
@@ -2047,8 +2049,9 @@ int fsvd_tile_model_create(const fsvd_dims* dims, const fsvd_layer* layers, cons
   if (ce == cudaSuccess) ce = cudaMalloc(&m->extra, extra);
   if (ce == cudaSuccess) ce = cudaMalloc(&m->xbuf[0], al256((size_t)D.B * D.d * 2));
   if (ce == cudaSuccess) ce = cudaMalloc(&m->xbuf[1], al256((size_t)D.B * D.d * 2));
-  if (ce == cudaSuccess) ce = clear_now(m->ws, m->L.total);
-  if (ce == cudaSuccess) ce = clear_now(m->extra, extra);
+  SideStream side;   // the clears run while the plans are made
+  if (ce == cudaSuccess) ce = side.clear(m->ws, m->L.total);
+  if (ce == cudaSuccess) ce = side.clear(m->extra, extra);
   if (ce != cudaSuccess) {
     fsvd_tile_model_destroy(m);
     return fail(FSVD_ERR_CUDA, "allocating model scratch failed");
@@ -2082,11 +2085,7 @@ int fsvd_tile_model_create(const fsvd_dims* dims, const fsvd_layer* layers, cons
     fsvd_tile_model_destroy(m);
     return launch_failed("cudaFuncSetAttribute failed for the tile kernel");
   }
-  cudaStream_t cs = nullptr;
-  if (cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking) != cudaSuccess) {
-    fsvd_tile_model_destroy(m);
-    return fail(FSVD_ERR_CUDA, "cudaStreamCreate failed");
-  }
+  const cudaStream_t cs = side.st;
   if (cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal) != cudaSuccess) e = fail(FSVD_ERR_CUDA, "stream capture failed");
   if (!e) {
     const long long before = fsvd_tile_launches();
@@ -2098,7 +2097,7 @@ int fsvd_tile_model_create(const fsvd_dims* dims, const fsvd_layer* layers, cons
     m->graph = g;
   }
   if (!e && cudaGraphInstantiate(&m->exec, m->graph, 0) != cudaSuccess) e = fail(FSVD_ERR_CUDA, "cudaGraphInstantiate failed");
-  cudaStreamDestroy(cs);
+  if (!e && side.wait() != cudaSuccess) e = fail(FSVD_ERR_CUDA, "clearing model scratch failed");
   if (e) {
     fsvd_tile_model_destroy(m);
     return e;
@@ -2218,7 +2217,8 @@ int fsvd_tile_prompt_create(const fsvd_dims* dims, const fsvd_layer* layers, con
   p->wait_limit = wait_limit;
   const size_t fixed = al256(sizeof(SyncState)) + al256((size_t)D.B * D.d * 2);
   cudaError_t ce = cudaMalloc(&p->fixed, fixed);
-  if (ce == cudaSuccess) ce = clear_now(p->fixed, fixed);
+  SideStream side;
+  if (ce == cudaSuccess) ce = side.clear(p->fixed, fixed);
   int e = ce == cudaSuccess ? prompt_scratch(p) : launch_failed("allocating prompt scratch failed");
   const int HD = D.H * D.Dh, KD = D.Hk * D.Dh;
   p->wmaps.resize((size_t)D.n_layers * PW_COUNT);
@@ -2235,6 +2235,7 @@ int fsvd_tile_prompt_create(const fsvd_dims* dims, const fsvd_layer* layers, con
     e = plan_gemm(p->head, lm_head, nullptr, D.vocab, D.d, D.d, prompt_last(p), nullptr, D.d, D.B, TE_STORE_F32, sc);
     p->head.a.out = p->logits;
   }
+  if (!e && side.wait() != cudaSuccess) e = launch_failed("clearing prompt scratch failed");
   if (e) {
     fsvd_tile_prompt_destroy(p);
     return e;
