@@ -236,12 +236,6 @@ static WsLayout ws_layout(const fsvd_dims& D) {
   return L;
 }
 
-// Running argmax keys of a model's rows (at most 8): behind the barrier words, in the same 256 bytes.
-static_assert(sizeof(SyncState) <= 128);
-static unsigned long long* argmax_keys(char* ws, const WsLayout& L) {
-  return reinterpret_cast<unsigned long long*>(ws + L.sync + 128);
-}
-
 // ------------------------------------------------------------------------------- builder
 struct MapPair {
   unsigned char m[2][128];
@@ -1247,7 +1241,6 @@ int fsvd_model_create(const fsvd_dims* dims, const fsvd_layer* layers, const voi
     s.flags = SF_OUT_T;
     s.tokens = m->tokens;
     s.vocab = D.vocab;
-    s.best = argmax_keys(m->ws, m->L);
     b.push(s);
   }
   for (int l = 0; l < D.n_layers; ++l) {
@@ -1262,13 +1255,13 @@ int fsvd_model_create(const fsvd_dims* dims, const fsvd_layer* layers, const voi
     s.eps = D.eps;
     s.epi = EPI_STORE;
     s.out = m->logits;
-    s.best = argmax_keys(m->ws, m->L);
+    s.best = argmax_keys(reinterpret_cast<SyncState*>(m->ws + m->L.sync));
   }
   {
     Stage s = b.blank();
     s.type = ST_ARGMAX;
     s.flags = 0;
-    s.best = argmax_keys(m->ws, m->L);
+    s.best = argmax_keys(reinterpret_cast<SyncState*>(m->ws + m->L.sync));
     s.vocab = D.vocab;
     s.tokens = m->tokens;
     s.token_log = m->token_log;
@@ -1414,7 +1407,7 @@ int fsvd_model_reset_sync(fsvd_model* m, void* stream) {
   if (!m) return fail(FSVD_ERR_ARG, "null model");
   if (m->prompt) return fsvd_workspace_clear_status(fsvd_tile_prompt_ws(m->prompt), stream);
   if (m->tile) return fsvd_tile_model_reset(m->tile, stream);
-  CUDA_TRY(cudaMemsetAsync(m->ws + m->L.sync, 0, sizeof(SyncState), (cudaStream_t)stream));
+  CUDA_TRY(cudaMemsetAsync(m->ws + m->L.sync, 0, al256(sizeof(SyncState)), (cudaStream_t)stream));   // (and the argmax keys)
   CUDA_TRY(cudaMemsetAsync(m->ws + m->L.counters, 0, kCounterBytes, (cudaStream_t)stream));
   return 0;
 }

@@ -1403,9 +1403,6 @@ template <typename T>
 __device__ __forceinline__ void run_embed(const Stage& st, int gtid, int gthreads) {
   using X = TT<T>;
   const int d = st.P, B = st.B;
-  // The keys of the step's argmax start at 0 here and not where the last step left them: in a step whose waits ran
-  // out, a CTA may have added to them after they were read.
-  if (st.best && gtid < B) st.best[gtid] = 0ull;
   for (int i = gtid; i < B * d; i += gthreads) {
     const int b = i / d, k = i - b * d;
     int tok = st.tokens[b];
@@ -1601,6 +1598,10 @@ fsvd_decode_kernel(const Stage* __restrict__ prog_global, const __grid_constant_
     if (done == gridDim.x - 1) {
       sync->done_ctas = 0;
       sync->arrivals = 0;
+      // The argmax keys of a model (at a fixed place behind these words) start every step at zero; here and not by the
+      // stage that reads them, because in a step whose waits ran out a CTA may add to them after that.
+      if (MODEL)
+        for (int b = 0; b < kArgmaxKeys; ++b) argmax_keys(sync)[b] = 0ull;
       sync->launches += 1;
     }
   }

@@ -102,7 +102,7 @@ struct alignas(16) Stage {
   int* step_counter;     // incremented once per ST_ARGMAX
   int* seqlens_rw;       // [B] incremented by ST_ARGMAX
   int vocab, max_steps;
-  unsigned long long* best;   // [B] running argmax keys of a model step: zeroed by ST_EMBED, raised by the lm_head stage, read by ST_ARGMAX; else null
+  unsigned long long* best;   // [B] running argmax keys of a model step: raised by the lm_head stage, read by ST_ARGMAX, zeroed by the launch's last CTA; else null
 };
 static_assert(sizeof(Stage) == 288, "Stage has no implicit padding");
 
@@ -115,6 +115,16 @@ struct SyncState {
   unsigned reserved;
   unsigned done_ctas;            // CTAs that have finished the running launch
 };
+
+// Running argmax keys of a model's rows: behind the barrier words, in the same 256 bytes.
+constexpr int kArgmaxKeys = 8;
+static_assert(sizeof(SyncState) <= 128);
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline unsigned long long* argmax_keys(SyncState* sync) {
+  return reinterpret_cast<unsigned long long*>(reinterpret_cast<char*>(sync) + 128);
+}
 
 enum DeviceStatus : int {
   DS_OK = 0,

@@ -71,12 +71,8 @@ def test_a_failed_launch_ends_a_prompt_pass():
 
 def test_argmax_keys_start_every_step_at_zero():
     """A step whose waits ran out leaves the argmax keys of its last CTAs behind; launches after it work
-    normally, so no step may begin with the keys of the one before."""
+    normally, so no step may begin with the keys of the one before: the last CTA of a launch zeroes them, after
+    every CTA has counted itself done."""
     kernel = (ROOT / "flashsvd_b200/csrc/fsvd_kernel.cuh").read_text()
-    embed = kernel[kernel.index("void run_embed("):]
-    embed = embed[:embed.index("\n}\n")]
-    assert "st.best[gtid] = 0ull" in embed
-    api = (ROOT / "flashsvd_b200/csrc/fsvd_api.cu").read_text()
-    for stage in ("ST_EMBED", "ST_ARGMAX"):
-        block = api[api.index(f"s.type = {stage};"):]
-        assert "s.best = argmax_keys(" in block[:block.index("b.push(s);")], stage
+    last = kernel[kernel.index("atomicAdd(&sync->done_ctas, 1u)"):]
+    assert "argmax_keys(sync)[b] = 0ull" in last and "__threadfence();" in kernel[kernel.index("if (*giveup)\n"):]
