@@ -92,6 +92,7 @@ class DecodeEngine:
         self.handle = handle
         self.max_steps = int(max_steps)
         self._pos_bound = 0   # host-side upper bound of the cache positions in use
+        self._seqlens_out = False   # the caller has been given a view of `seqlens` and may write through it at any time
         # Prompt of a single fp32 or int4 sequence: a second program over the same weights and caches takes
         # `prefill_chunk` consecutive prompt positions per launch (rows_are_positions of fsvd_dims);
         # it is created on the first prompt that is long enough.  For bf16, where the prompt program below takes
@@ -122,8 +123,12 @@ class DecodeEngine:
     @property
     def seqlens(self):
         # the caller may write through this view: the host-side position bound is no longer known
-        self._pos_bound = None
+        self._pos_bound, self._seqlens_out = None, True
         return self._view("seqlens", (self.B,), torch.int32)
+
+    def _fill_positions(self, value: int) -> None:
+        self._view("seqlens", (self.B,), torch.int32).fill_(int(value))
+        self._pos_bound = int(value)
 
     @property
     def token_log(self):
@@ -156,9 +161,8 @@ class DecodeEngine:
         check(self.lib.fsvd_model_step(self.handle, int(n_steps), torch.cuda.current_stream().cuda_stream))
 
     def reset(self) -> None:
-        self.seqlens.zero_()
+        self._fill_positions(0)
         self.step_counter.zero_()
-        self._pos_bound = 0
 
     def _chunk_model(self):
         """The program that takes `prefill_chunk` prompt positions of the one sequence per launch; returns
@@ -208,9 +212,12 @@ class DecodeEngine:
         Cn = self.prefill_chunk
         stream = torch.cuda.current_stream().cuda_stream
         if self.B == 1 and L > Cn > 1:
-            # the position on the device: the host's bound does not know of a write through a view of
-            # `seqlens` that the caller has kept
-            pos0 = self._pos_bound = int(self._view("seqlens", (1,), torch.int32).item())
+            # The position on the device, wherever the host's may not be the same: it does not know of a write through
+            # a view of `seqlens`, and chunks start where it says.  (The prompt program takes its positions from the
+            # device; the read costs 20 us of a short prompt.)
+            if self._seqlens_out or self._pos_bound is None or not self.prefill_tile:
+                self._pos_bound = int(self._view("seqlens", (1,), torch.int32).item())
+            pos0 = self._pos_bound
             if pos0 + L > self.S_max:
                 raise ValueError(f"prompt of {L} tokens at position {pos0} exceeds the cache ({self.S_max})")
         # (its program is made by the first prompt, which allocates: a first prompt inside a graph capture goes
@@ -228,8 +235,7 @@ class DecodeEngine:
                 seqlens.copy_(offs + (pos0 + t0))
                 check(self.lib.fsvd_model_step(handle, 1, stream))
                 t0 += Cn
-            self.seqlens.fill_(pos0 + t0)
-            self._pos_bound = pos0 + t0
+            self._fill_positions(pos0 + t0)
         tok = self.tokens
         for t in range(t0, L):
             tok.copy_(prompt[:, t])
@@ -405,8 +411,7 @@ class EngineGroup:
 
     def fill_seqlens(self, value: int) -> None:
         for e in self.engines:
-            e.seqlens.fill_(int(value))
-            e._pos_bound = int(value)
+            e._fill_positions(value)
 
     def step(self, n_steps: int = 1) -> None:
         for _ in range(int(n_steps)):

@@ -101,6 +101,13 @@ def test_prompt_starts_where_the_device_says(dtype):
     w = O.make_model_weights(shape, seed=6, dtype=dtype)
     first, second = torch.randint(0, shape.vocab, (2, 1, L), generator=torch.Generator().manual_seed(4))
     ref = _engine(shape, w, 1, L + 4)
+    ref.prefill(first[:, :13])
+    ref.step(2)
+    with pytest.raises((IndexError, ValueError)):
+        ref.prefill(second)             # 15 + 21 positions, nobody holds a view
+    ref.reset()
+    for c in (*ref.key_cache, *ref.value_cache):
+        c.zero_()
     ref.prefill(second)
     eng = _engine(shape, w, 1, L + 4)
     lens = eng.seqlens
