@@ -329,7 +329,7 @@ __global__ void __launch_bounds__(kPgThreads, 1) prompt_gemm_kernel(const __grid
 // (they decide the first token), by CTAs of their own in front of the others: 16 query vectors, the key blocks dealt
 // out to the four warps, which are through long before a block of 64 with as many keys.  The earlier rows are bound
 // by mma.sync: 2041 positions through 4 layers of 32 heads of 128 take 2.80 ms with no FULL row, 2.77 like this, 2.90 with
-// the last block of 64 rows FULL and 3.12 with all of them; 4 prompts of 180 (all FULL) 1.37 and 1.40 ms.
+// the last block of 64 rows FULL and 3.12 with all of them; 4 prompts of 180 (all FULL) 1.39 and 1.40 ms.
 constexpr int kPaWarps = 4;
 constexpr int kPaSlots = 16 * kPaWarps;
 constexpr int kPaKeys = 64;
@@ -685,8 +685,10 @@ __device__ __forceinline__ void prompt_attn_tail(const PaArgs& a, unsigned char*
   }
 }
 
+// (FULL: a CTA less per SM and no spills in the loop; 2 prompts of 100 positions, 4 layers of 32 heads of 128 1183 -> 1161 us, as
+// without full weights)
 template <int DH, bool FULL>
-__global__ void __launch_bounds__(kPaWarps * 32, DH == 64 ? 4 : 3) prompt_attn_kernel(const PaArgs a) {
+__global__ void __launch_bounds__(kPaWarps * 32, (DH == 64 ? 4 : 3) - (FULL ? 1 : 0)) prompt_attn_kernel(const PaArgs a) {
   extern __shared__ __align__(16) unsigned char pa_smem[];
   pdl_launch_dependents();
   pdl_wait();
