@@ -1358,6 +1358,7 @@ int fsvd_prompt_create(const fsvd_dims* dims, const fsvd_layer* layers, const vo
   fsvd_tile_decode_state st;
   memset(&st, 0, sizeof(st));
   if (int e = fsvd_model_buffers(decode, &st.tokens, &st.seqlens, &st.token_log, &st.step_counter, &st.logits, nullptr)) return e;
+  st.ws = decode->tile ? fsvd_tile_model_ws(decode->tile) : decode->ws + decode->L.sync;
   st.max_steps = decode->max_steps < 1 ? 1 : decode->max_steps;
   fsvd_tile_prompt* p = nullptr;
   if (int e = fsvd_tile_prompt_create(dims, layers, embed, final_norm_w, lm_head, cos_tab, sin_tab, &st,

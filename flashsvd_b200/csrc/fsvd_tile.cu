@@ -2150,19 +2150,17 @@ struct fsvd_tile_prompt {
   float* logits = nullptr;
   int max_steps = 0;
   long long wait_limit = 0;
-  char* fixed = nullptr;             // status words, normalised last rows
+  SyncState* sync = nullptr;         // the decode model's
+  __nv_bfloat16* last = nullptr;     // normalised last rows
   char* ws = nullptr;                // rows of everything below
   int *rowpos = nullptr, *rowseq = nullptr;
   __nv_bfloat16 *x = nullptr, *mid = nullptr, *xn = nullptr, *pbuf = nullptr, *qbuf = nullptr, *attn = nullptr, *hact = nullptr;
   GemmPlan head;
 };
 
-static SyncState* prompt_sync(fsvd_tile_prompt* p) { return reinterpret_cast<SyncState*>(p->fixed); }
-static __nv_bfloat16* prompt_last(fsvd_tile_prompt* p) { return reinterpret_cast<__nv_bfloat16*>(p->fixed + al256(sizeof(SyncState))); }
-
 int fsvd_tile_prompt_destroy(fsvd_tile_prompt* p) {
   if (!p) return 0;
-  cudaFree(p->fixed);
+  cudaFree(p->last);
   cudaFree(p->ws);
   delete p;
   return 0;
@@ -2215,11 +2213,8 @@ int fsvd_tile_prompt_create(const fsvd_dims* dims, const fsvd_layer* layers, con
   p->logits = st->logits;
   p->max_steps = st->max_steps;
   p->wait_limit = wait_limit;
-  const size_t fixed = al256(sizeof(SyncState)) + al256((size_t)D.B * D.d * 2);
-  cudaError_t ce = cudaMalloc(&p->fixed, fixed);
-  SideStream side;
-  if (ce == cudaSuccess) ce = side.clear(p->fixed, fixed);
-  int e = ce == cudaSuccess ? prompt_scratch(p) : launch_failed("allocating prompt scratch failed");
+  p->sync = reinterpret_cast<SyncState*>(st->ws);
+  int e = cudaMalloc(&p->last, (size_t)D.B * D.d * 2) == cudaSuccess ? prompt_scratch(p) : launch_failed("allocating prompt scratch failed");
   const int HD = D.H * D.Dh, KD = D.Hk * D.Dh;
   p->wmaps.resize((size_t)D.n_layers * PW_COUNT);
   for (int l = 0; l < D.n_layers && !e; ++l) {
@@ -2231,11 +2226,10 @@ int fsvd_tile_prompt_create(const fsvd_dims* dims, const fsvd_layer* layers, con
     for (int i = 0; i < PW_COUNT && !e; ++i) e = encode_sw128(&m[i], f[i].base, f[i].rows, f[i].K, f[i].K, kPgBoxRows);
   }
   if (!e) {
-    Scratch sc = {&prompt_sync(p)->status, wait_limit};
-    e = plan_gemm(p->head, lm_head, nullptr, D.vocab, D.d, D.d, prompt_last(p), nullptr, D.d, D.B, TE_STORE_F32, sc);
+    Scratch sc = {&p->sync->status, wait_limit};
+    e = plan_gemm(p->head, lm_head, nullptr, D.vocab, D.d, D.d, p->last, nullptr, D.d, D.B, TE_STORE_F32, sc);
     p->head.a.out = p->logits;
   }
-  if (!e && side.wait() != cudaSuccess) e = launch_failed("clearing prompt scratch failed");
   if (e) {
     fsvd_tile_prompt_destroy(p);
     return e;
@@ -2281,7 +2275,7 @@ static int launch_prompt_gemm(fsvd_tile_prompt* p, int layer, const PgSpec* sp, 
   a.tiles_m = (rows + kTileM - 1) / kTileM;
   a.rowpos = p->rowpos; a.rowseq = p->rowseq; a.cos_tab = p->cos_tab; a.sin_tab = p->sin_tab;
   a.Dh = D.Dh; a.HkDh = D.Hk * D.Dh; a.S_max = D.S_max;
-  a.status = &prompt_sync(p)->status;
+  a.status = &p->sync->status;
   a.wait_limit = p->wait_limit;
   const bool two = sp[0].w2 >= 0;
   const bool rope = sp[0].epi == TE_ROPE_Q;
@@ -2370,7 +2364,7 @@ int fsvd_tile_prompt_run(fsvd_tile_prompt* p, const int* prompt, int ld, int L, 
       continue;
     }
     // the last position of every sequence: final norm, head, argmax
-    norm(p->x, p->final_norm, prompt_last(p), D.B, n, n - 1);
+    norm(p->x, p->final_norm, p->last, D.B, n, n - 1);
     if (!e) e = launch_gemm(p->head, st);
     if (!e)
       launched(launch_pdl(argmax_rows_kernel, dim3(D.B), dim3(256), 0, st, (const float*)p->logits, D.vocab, p->tokens, p->token_log,
@@ -2379,7 +2373,7 @@ int fsvd_tile_prompt_run(fsvd_tile_prompt* p, const int* prompt, int ld, int L, 
   }
   return e;
 }
-void* fsvd_tile_prompt_ws(fsvd_tile_prompt* p) { return p->fixed; }
+void* fsvd_tile_prompt_ws(fsvd_tile_prompt* p) { return p->sync; }
 
 // Debugging aid: while a device buffer is set, every GEMM CTA planned afterwards records nine
 // %globaltimer marks (entry, set-up done, dependency met, accumulators done, cluster barrier 1,

@@ -40,8 +40,9 @@ int fsvd_tile_model_launches_per_step(fsvd_tile_model* m);
 int fsvd_tile_model_reset(fsvd_tile_model* m, void* stream);
 
 // Prompt pass over the weights and caches of a decode model: reads and advances its positions, leaves the
-// last position's token and logits in its buffers.
+// last position's token and logits in its buffers, reports in its status word.
 struct fsvd_tile_decode_state {
+  void* ws;   // starts with the decode model's SyncState
   int *tokens, *seqlens, *step_counter, *token_log;
   float* logits;
   int max_steps;

@@ -250,8 +250,9 @@ int fsvd_model_step(fsvd_model* m, int n_steps, void* stream);
  * caches, and leaves the token sampled after the last position in the decode model's tokens / token_log,
  * its logits in logits, and seqlens / step_counter advanced by length / 1.  The scratch of min(2048, B S_max)
  * rows (2048 rows of a 7B shape: 140 MB) is allocated by fsvd_prompt_create and freed by fsvd_model_destroy; a run
- * allocates nothing and can be captured into a graph.  fsvd_model_status, fsvd_model_reset_sync
- * and fsvd_model_destroy take a prompt program too; it is destroyed before the decode model.  The
+ * allocates nothing and can be captured into a graph.  The program reports in the decode model's status word.
+ * fsvd_model_status, fsvd_model_reset_sync and fsvd_model_destroy take a prompt program too; it is destroyed before
+ * the decode model.  The
  * reference fills the cache with its prefill kernels (kernels/flashsvdropeattn.py:67-427). */
 int fsvd_prompt_create(const fsvd_dims* dims, const fsvd_layer* layers, const void* embed,
                        const void* final_norm_w, const void* lm_head, const void* cos_tab,
