@@ -255,8 +255,8 @@ def time_workload(dev, *, shape_name, layers, batch, ctx, share_pairs, factors, 
 
 
 def time_prefill(dev, lengths, seed=0):
-    """Prompt pass of one sequence through the 32-layer 7B-shape model (128 positions per pass on the
-    tiled tensor-core path, the tail in smaller passes): ms per prompt and prompt tokens/s."""
+    """Prompt pass of one sequence through the 32-layer 7B-shape model (all positions as the rows of the prompt
+    program's tensor-core GEMMs, up to 2048 per pass): ms per prompt and prompt tokens/s."""
     import torch
 
     from flashsvd_b200 import synthetic
@@ -268,7 +268,7 @@ def time_prefill(dev, lengths, seed=0):
     gen = torch.Generator(device=dev).manual_seed(seed)
     for L in lengths:
         prompt = torch.randint(0, shape.vocab, (1, L), device=dev, generator=gen, dtype=torch.int32)
-        for it in range(2):      # the first pass builds the 128-row program (CUDA graph capture)
+        for it in range(2):      # the first pass builds the prompt program and its scratch
             eng.reset()
             torch.cuda.synchronize()
             e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
